@@ -313,15 +313,14 @@ int qtb_plan_run_plain(qtb_plan* plan, int32_t first, int32_t count, const doubl
  * memory, classes concurrent) with 64..1024 threads per CTA, then the whole
  * class schedule against the persistent, hybrid (large networks as
  * classes + a lean persistent queue) and warp-per-network schedules, and
- * keeps the fastest; with wide networks it then times the wave kernel with
- * 8 and with 4 elements per thread in flight and keeps the faster; later
- * runs reuse the choices.
+ * keeps the fastest; later runs reuse the choices.  A range with wide
+ * networks keeps the class schedule and its default block sizes: their
+ * waves outlast the other networks' launches.
  * QTB_AUTOTUNE=0 in the environment keeps the default block sizes;
- * QTB_SCHEDULE and QTB_WIDE_BATCH (2 or 3) fix the schedule and the wave
- * variant.                                                               */
+ * QTB_SCHEDULE fixes the schedule.                                       */
 int qtb_plan_set_autotune(qtb_plan* plan, int32_t enable);
-/* Resident CTAs per SM of the plan's wide waves (0, the default: as many
- * as fit, two).  A wave keeps its CTAs for its whole run; with 1, half of
+/* Halves of every SM that the plan's wide waves may hold (0, the default:
+ * both; a half is two CTAs of 256 threads).  A wave keeps its CTAs for its whole run; with 1, half of
  * every SM stays free for other streams' kernels (a server's concurrent
  * requests) while a wide request runs.  Set before a range's first run.  */
 int qtb_plan_set_wave_ctas_per_sm(qtb_plan* plan, int32_t ctas);

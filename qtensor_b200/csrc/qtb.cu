@@ -377,6 +377,11 @@ __device__ void reduce_energy(const float2* terms, uint32_t n, double n_groups, 
     __syncthreads();
 }
 
+// The same out of line, for kernels whose registers are counted.
+__device__ __noinline__ void reduce_energy_call(const float2* terms, uint32_t n, double n_groups, double* energy) {
+    reduce_energy(terms, n, n_groups, energy);
+}
+
 // The op of a phase holding flattened element g, starting from op `oi` at
 // or before it (`op` holds ops[oi]).  The ops of a phase are sorted by
 // non-increasing size, so jumping (g - start) >> w ops ahead never passes
@@ -1013,13 +1018,18 @@ __global__ void __launch_bounds__(kWarpMaxThreads) qtb_warp_network_kernel(const
 
 // ----------------------------------------------------------------- K4
 // Wide networks (arenas too large for shared memory) are contracted by the
-// whole GPU at once.  The networks of a wave advance together, one step per
-// elimination phase: step s holds phase s of every wave network that has
-// one, its elements concatenated (segments) and cut into tiles.  CTAs claim
-// tiles in order from a queue; a tile of step s starts once every tile of
-// step s-1 has finished.  A CTA only ever waits for tiles that were claimed
-// before its own, i.e. by CTAs that are running, so the scheme needs no
-// co-residency guarantee (no cooperative launch), and every wait is bounded.
+// whole GPU at once.  Every phase of every network of a wave is cut into
+// items -- one per large op, one per run of small ops, one per run of whole
+// phases too small to split -- and every item into tiles.  Tiles whose
+// network has finished the previous phase are in a queue; CTAs take tickets
+// for its places in order and wait for their place to be filled.  The CTA
+// that finishes a phase's last tile (one counter per network and phase)
+// queues the tiles of the network's next phase, so every network advances
+// at its own pace and a CTA only waits when no tile at all is ready.
+// A ticket's place is filled by the tiles that running CTAs hold, and a CTA
+// holds a second ticket only while the place of that ticket is filled
+// already, so the scheme needs no co-residency guarantee (no cooperative
+// launch), and every wait is bounded.
 struct WideNet {
     const DevNetRun* run;
     float2* term;
@@ -1027,50 +1037,70 @@ struct WideNet {
     uint64_t pad;
 };
 
-struct WideStep {
-    uint32_t seg_begin;     // into the wave's segments
-    uint32_t n_segs;
-    uint32_t tile_begin;    // first tile of the step
-    uint32_t n_tiles;
-    uint32_t total_elems;
-    uint32_t tile_elems;    // elements per tile of this step (a multiple of 4 x block size)
-    uint32_t pad[2];
+struct WideItem {
+    uint64_t arena_off;     // the network's arena, complex64 elements into the wave's arenas
+    uint64_t plan_off;      // bytes into the plan blobs: the network's ops (kWideOp: the op's operands)
+    uint32_t a;             // the network's operands, bytes after its ops (kWideOp: the op's output)
+    uint32_t begin, end;    // its ops (kWideChain: its phases; kWideOp: output variables | operands << 8 | sum << 16)
+    uint32_t elem_begin;    // elements of the phase that it covers (kWideChain: the network's phases)
+    uint32_t elem_end;
+    uint32_t tile_elems;    // elements per tile
+    uint32_t done;          // counter of its phase
+    uint32_t need;          // tiles of its phase
+    uint32_t next;          // items and tiles of the network's next phase
+    uint32_t next_items;
+    uint32_t next_tiles;
+    uint32_t kind_net;      // kind | last phase << 2 | network << 3
 };
 
-struct WideSeg {
-    uint32_t net;           // wave-local network
-    uint32_t elem_begin;    // first element of the network's phase within the step
-};
+constexpr uint32_t kWideOp = 0;      // one op of at least kWideChunk elements
+constexpr uint32_t kWideSmall = 1;   // a run of ops of one phase
+constexpr uint32_t kWideChain = 2;   // whole phases, one tile: the CTA's barriers separate them
 
 struct WideArgs {
     const WideNet* nets;
-    const WideStep* steps;
-    const WideSeg* segs;
-    unsigned int* counters;   // [0] next tile, [1 + s] finished tiles of step s (zeroed per launch)
+    const WideItem* items;
+    // zeroed per launch: [0] tickets taken, [1] places filled by finished
+    // phases, then the finished tiles of every network and phase
+    unsigned int* counters;
+    // the places after the first n_ready: (item + 1) << 32 | tile of the
+    // item, 0 while empty (zeroed per launch)
+    unsigned long long* queue;
+    const unsigned long long* ready;   // the first n_ready places: every network's first phase
     float2* arenas;
-    uint32_t n_nets;
-    uint32_t n_steps;
-    uint32_t n_tiles;         // tile n_tiles (the last one) writes the wave's terms
+    uint32_t n_tiles;
+    uint32_t n_ready;
+    uint32_t vec;                // arenas are 16-byte aligned
 };
 
 static_assert(sizeof(WideNet) == 32, "WideNet layout");
-static_assert(sizeof(WideStep) == 32, "WideStep layout");
+static_assert(sizeof(WideItem) == 64, "WideItem layout");
 constexpr uint32_t kWideSpinLimit = 1u << 23;   // about 1 s of polling
 constexpr int kWideThreads = 256;
-// log2 of the elements a thread has in flight: the wave kernel comes in
-// two variants, 8 (3) and 4 (2) elements, chosen per plan by the autotuner
-// (the smaller batch needs fewer registers and won on N=256 p=4, the larger
-// on Erdos-Renyi N=400 p=3)
-constexpr uint32_t kWideBatchLog = 3;
-constexpr uint32_t kWideBatch = 1u << kWideBatchLog;
-constexpr uint32_t kWideGroup = 1;                                  // operands per batch of loads
-constexpr uint32_t kWideMinTile = kWideBatch * kWideThreads;         // 2048
-constexpr uint32_t kWideMaxTile = 8 * kWideMinTile;
+constexpr int kWideCtasPerSm = 4;                       // 64 registers per thread
+constexpr uint32_t kWideChunk = 4 * kWideThreads;       // elements of an op that a CTA contracts at once
+constexpr uint32_t kWideMaxK = 16;                      // operands of a kWideOp item
+constexpr uint32_t kWideGroup = 16;                     // chunks whose operand addresses are prepared at once
+constexpr uint32_t kWideMaxTileChunks = 64;
+constexpr uint32_t kWideSmallElems = 2;                 // elements per thread and pass of small ops
+constexpr uint32_t kWideSmallTile = kWideSmallElems * kWideThreads;
+constexpr uint32_t kWideChainElems = 512;               // largest phase of a chain
+constexpr uint32_t kWideSmemOps = 2048;                 // ops whose first elements a tile keeps in shared memory
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
+}
+
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_release64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Bounded wait until *counter reaches need (acquire).  Returns false after
@@ -1151,13 +1181,12 @@ __device__ __forceinline__ void compute_element_wide(const DevOp& op, uint32_t j
     arena[op.dst + j] = op.sum ? make_float2(p0.x + p1.x, p0.y + p1.y) : p0;
 }
 
-// 2^kBatchLog elements j + 256 e of one op at once, with the kBatchLog
-// bits of j from bit 8 up zero: they differ from j only in those bits, so
-// each operand offset is the gathered offset of j plus the gathered offsets
-// of those bits (one full gather per operand, not one per element), and the
-// loads of kWideGroup operands for all elements are issued together
-// (2^(kBatchLog + 1) L2 requests in flight per thread and operand).
-template <uint32_t kBatchLog>
+// Eight elements j + 256 e of one op at once, with bits 8-10 of j zero: they
+// differ from j only in those bits, so each operand offset is the gathered
+// offset of j plus the gathered offsets of those bits (one full gather per
+// operand, not one per element), and an operand's loads for all elements
+// are issued together.
+constexpr uint32_t kBatchLog = 3;
 __device__ __forceinline__ void compute_elements_wide(const DevOp& op, uint32_t j, const DevIn* ins,
                                                        const float2* __restrict__ table,
                                                        float2* __restrict__ arena) {
@@ -1168,52 +1197,33 @@ __device__ __forceinline__ void compute_elements_wide(const DevOp& op, uint32_t 
     float2 p0[kB], p1[kB];
 #pragma unroll
     for (uint32_t e = 0; e < kB; ++e) p0[e] = p1[e] = make_float2(1.f, 0.f);
-    for (uint32_t t0 = 0; t0 < op.k; t0 += kWideGroup) {
-        DevIn d[kWideGroup];
+    for (uint32_t t = 0; t < op.k; ++t) {
+        const DevIn d = ldg_in(in + t);
+        const bool tab = d.src & kSrcTable;
+        const float2* base = tab ? table + (d.src & ~kSrcTable) : arena + d.src;
+        const bool has_sum = op.sum && ((d.mask >> w) & 1u);
+        const uint32_t stride_s = has_sum ? 1u << (__popc(d.mask) - 1) : 0u;
+        const uint32_t m = d.mask & low;
+        // bit 8 + i of j lands at operand bit popc(m below it) when m has it
+        uint32_t bit_off[kBatchLog];
 #pragma unroll
-        for (int t = 0; t < kWideGroup; ++t)
-            if (t0 + t < op.k) d[t] = ldg_in(in + t0 + t);
-        float2 x0[kWideGroup][kB], x1[kWideGroup][kB];
+        for (uint32_t i = 0; i < kBatchLog; ++i)
+            bit_off[i] = ((m >> (8 + i)) & 1u) << __popc(m & ((1u << (8 + i)) - 1u));
+        const uint32_t off = gather_bits(j, d, low);
+        float2 x0[kB], x1[kB];
 #pragma unroll
-        for (int t = 0; t < kWideGroup; ++t) {
-            if (t0 + t < op.k) {
-                const bool tab = d[t].src & kSrcTable;
-                const float2* base = tab ? table + (d[t].src & ~kSrcTable) : arena + d[t].src;
-                const bool has_sum = op.sum && ((d[t].mask >> w) & 1u);
-                const uint32_t stride_s = has_sum ? 1u << (__popc(d[t].mask) - 1) : 0u;
-                const uint32_t m = d[t].mask & low;
-                // bit 8 + i of j lands at operand bit popc(m below it) when m has it
-                uint32_t bit_off[kBatchLog];
+        for (uint32_t e = 0; e < kB; ++e) {
+            uint32_t o = off;
 #pragma unroll
-                for (uint32_t i = 0; i < kBatchLog; ++i)
-                    bit_off[i] = ((m >> (8 + i)) & 1u) << __popc(m & ((1u << (8 + i)) - 1u));
-                uint32_t off[kB];
-                off[0] = gather_bits(j, d[t], low);
-#pragma unroll
-                for (uint32_t e = 1; e < kB; ++e) {
-                    uint32_t o = off[0];
-#pragma unroll
-                    for (uint32_t i = 0; i < kBatchLog; ++i)
-                        if ((e >> i) & 1u) o += bit_off[i];
-                    off[e] = o;
-                }
-#pragma unroll
-                for (uint32_t e = 0; e < kB; ++e) {
-                    x0[t][e] = tab ? __ldg(base + off[e]) : __ldcg(base + off[e]);
-                    x1[t][e] = has_sum ? (tab ? __ldg(base + off[e] + stride_s) : __ldcg(base + off[e] + stride_s))
-                                       : x0[t][e];
-                }
-            }
+            for (uint32_t i = 0; i < kBatchLog; ++i)
+                if ((e >> i) & 1u) o += bit_off[i];
+            x0[e] = tab ? __ldg(base + o) : __ldcg(base + o);
+            x1[e] = has_sum ? (tab ? __ldg(base + o + stride_s) : __ldcg(base + o + stride_s)) : x0[e];
         }
 #pragma unroll
-        for (int t = 0; t < kWideGroup; ++t) {
-            if (t0 + t < op.k) {
-#pragma unroll
-                for (uint32_t e = 0; e < kB; ++e) {
-                    p0[e] = cmul(p0[e], x0[t][e]);
-                    p1[e] = cmul(p1[e], x1[t][e]);
-                }
-            }
+        for (uint32_t e = 0; e < kB; ++e) {
+            p0[e] = cmul(p0[e], x0[e]);
+            p1[e] = cmul(p1[e], x1[e]);
         }
     }
 #pragma unroll
@@ -1221,129 +1231,342 @@ __device__ __forceinline__ void compute_elements_wide(const DevOp& op, uint32_t 
         arena[op.dst + j + e * 256u] = op.sum ? make_float2(p0[e].x + p1[e].x, p0[e].y + p1[e].y) : p0[e];
 }
 
-template <uint32_t kBatchLog>
-__global__ void __launch_bounds__(kWideThreads, 2) qtb_wide_kernel(const WideArgs w, const RunArgs a) {
-    constexpr uint32_t kB = 1u << kBatchLog;
-    constexpr uint32_t kBatchBits = (kB - 1u) << 8;   // the bits of j above the thread index
-    __shared__ uint32_t s_tile;
-    __shared__ int s_ok, s_last;
+// Elements g0, g0 + 256, ... (kWideSmallElems of them, below g_end) of ops
+// lo .. hi - 1 of a phase, whatever their sizes: each element finds its op by
+// binary search over the ops' first elements (`first` in shared memory, or
+// null: the ops are too many) and gathers each operand's offset for itself.  The elements
+// of a thread go through every dependent load (op search, op, operand
+// descriptor, operand) together, so that their latencies overlap.
+__device__ __forceinline__ void wide_small(const DevOp* ops, uint32_t lo, uint32_t hi, uint32_t g0, uint32_t g_end,
+                                           const uint32_t* first, const DevIn* ins, const float2* table,
+                                           float2* arena) {
+    constexpr uint32_t E = kWideSmallElems;
+    uint32_t at[E], g[E];
+#pragma unroll
+    for (uint32_t i = 0; i < E; ++i) {
+        at[i] = lo;
+        g[i] = min(g0 + i * kWideThreads, g_end - 1u);
+    }
+    for (uint32_t size = hi - lo; size > 1u;) {
+        const uint32_t half = size >> 1;
+#pragma unroll
+        for (uint32_t i = 0; i < E; ++i)
+            if ((first ? first[at[i] - lo + half] : __ldg(&ops[at[i] + half].elem_begin)) <= g[i]) at[i] += half;
+        size -= half;
+    }
+    uint32_t j[E], dst[E], uk[E];
+    const DevIn* in[E];
+    uint32_t kmax = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < E; ++i) {
+        const DevOp op = ldg_op(ops + at[i]);
+        j[i] = g[i] - op.elem_begin;
+        dst[i] = op.dst + j[i];
+        in[i] = ins + op.in_begin;
+        uk[i] = (uint32_t)op.k | (op.sum ? 0x100u : 0u) | (uint32_t)(op.u - op.sum) << 16;
+        kmax = max(kmax, (uint32_t)op.k);
+    }
+    float2 p0[E], p1[E];
+#pragma unroll 1
+    for (uint32_t t = 0; t < kmax; ++t) {
+        float2 x0[E], x1[E];
+#pragma unroll
+        for (uint32_t i = 0; i < E; ++i)
+            if (t < (uk[i] & 0xffu)) {
+                const DevIn d = ldg_in(in[i] + t);
+                const uint32_t w = uk[i] >> 16;
+                const float2* x = ((d.src & kSrcTable) ? table + (d.src & ~kSrcTable) : arena + d.src) +
+                                  gather_bits(j[i], d, (1u << w) - 1u);
+                const bool has = (uk[i] & 0x100u) && ((d.mask >> w) & 1u);
+                x0[i] = *x;
+                x1[i] = has ? x[1u << (__popc(d.mask) - 1)] : x0[i];
+            }
+#pragma unroll
+        for (uint32_t i = 0; i < E; ++i)
+            if (t < (uk[i] & 0xffu)) {
+                p0[i] = t == 0 ? x0[i] : cmul(p0[i], x0[i]);
+                p1[i] = t == 0 ? x1[i] : cmul(p1[i], x1[i]);
+            }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < E; ++i)
+        if (g0 + i * kWideThreads < g_end)
+            arena[dst[i]] = (uk[i] & 0x100u) ? make_float2(p0[i].x + p1[i].x, p0[i].y + p1[i].y) : p0[i];
+}
+
+// An operand of a kWideOp item: where its offset moves with the bits that
+// are not in the thread's gathered offset.
+struct WideOperand {
+    uint32_t sum;    // stride of the summed variable (0: the operand lacks it)
+    uint32_t hi;     // stride of element bit 9
+    uint32_t lo;     // stride of element bit 0 (0 or 1)
+    uint32_t pair;   // bits 0 and the base allow 16-byte loads of element pairs
+};
+
+// The four elements of a thread (bits 0 and 9 of the element index) of one
+// operand at p, for the summed variable at 0 (x0) and at 1 (x1).  Every load
+// is issued before any value is used: a stride of 0 loads the same address
+// again (an L1 hit) rather than wait for a value to copy.  The branches are
+// uniform.
+__device__ __forceinline__ void wide_load(const float2* p, const WideOperand& o, float2 (&x0)[4], float2 (&x1)[4]) {
+    __builtin_assume(__isGlobal(p));
+    const float2* const q[4] = {p, p + o.hi, p + o.sum, p + o.sum + o.hi};
+    if (o.pair) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(q[i]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            x0[2 * i] = make_float2(v[i].x, v[i].y);
+            x0[2 * i + 1] = make_float2(v[i].z, v[i].w);
+            x1[2 * i] = make_float2(v[2 + i].x, v[2 + i].y);
+            x1[2 * i + 1] = make_float2(v[2 + i].z, v[2 + i].w);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            x0[2 * i] = *q[i];
+            x1[2 * i] = *q[2 + i];
+        }
+        if (o.lo) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                x0[2 * i + 1] = q[i][1];
+                x1[2 * i + 1] = q[2 + i][1];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                x0[2 * i + 1] = x0[2 * i];
+                x1[2 * i + 1] = x1[2 * i];
+            }
+        }
+    }
+}
+
+// What a tile prepares in shared memory for its op.  An operand's offset is
+// a sum over disjoint bits of the element index: the parts of the lane (bits
+// 1-5) and of the warp (bits 6-8), bits 0 and 9 (WideOperand), and the
+// chunk's part, which the chunk's address holds.
+struct WideShared {
+    union {
+        struct {
+            const float2* ptr[kWideMaxK][kWideGroup];
+            uint16_t lane[kWideMaxK][32];
+            uint16_t warp[kWideMaxK][kWideThreads / 32];
+            WideOperand meta[kWideMaxK];
+            uint16_t off[kWideMaxK][kWideThreads];   // the thread's: lane + warp
+        };
+        uint32_t op_first[kWideSmemOps];   // small ops
+    };
+    unsigned long long place;   // of the tile to run; 0: no tile left, or the wait ran out
+    uint32_t finished, first_place, last;
+};
+
+// Addresses of `chunks` chunks of an op's operands from element j0 on, and
+// with `all` the parts of the offsets that do not change from chunk to chunk;
+// about one gather per thread for four operands.
+__device__ __forceinline__ void wide_prepare(WideShared& s, const DevIn* in, uint32_t k, uint32_t ow, bool sum,
+                                             uint32_t j0, uint32_t chunks, bool all, bool vec, const float2* table,
+                                             const float2* arena) {
+    const uint32_t low = (1u << ow) - 1u;
+    const uint32_t fixed = all ? 32u + kWideThreads / 32u + 1u : 0u, each = fixed + chunks;
+    for (uint32_t i = threadIdx.x; i < k * each; i += kWideThreads) {
+        const uint32_t q = i / each, r = i % each;
+        const DevIn d = ldg_in(in + q);
+        if (r >= fixed) {
+            s.ptr[q][r - fixed] = ((d.src & kSrcTable) ? table + (d.src & ~kSrcTable) : arena + d.src) +
+                                  gather_bits(j0 + (r - fixed) * kWideChunk, d, low);
+        } else if (r < 32u) {
+            s.lane[q][r] = (uint16_t)gather_bits(r << 1, d, low);
+        } else if (r < fixed - 1u) {
+            s.warp[q][r - 32u] = (uint16_t)gather_bits((r - 32u) << 6, d, low);
+        } else {
+            WideOperand o;
+            o.sum = (sum && ((d.mask >> ow) & 1u)) ? 1u << (__popc(d.mask) - 1) : 0u;
+            o.hi = ((d.mask >> 9) & 1u) << __popc(d.mask & 0x1ffu);
+            o.lo = d.mask & 1u;
+            // arena tensors start at multiples of four elements; a gate
+            // table entry may start anywhere
+            o.pair = o.lo && vec && !(d.src & kSrcTable);
+            s.meta[q] = o;
+        }
+    }
+}
+
+// The place of ticket t (one thread; bounded wait until it is filled).
+__device__ unsigned long long wide_place(const WideArgs& w, uint32_t t, int* status) {
+    if (t >= w.n_tiles) return 0ull;
+    if (t < w.n_ready) return w.ready[t];
+    const unsigned long long* p = w.queue + (t - w.n_ready);
+    unsigned long long v;
+    for (uint32_t it = 0; (v = ld_acquire64(p)) == 0ull;) {
+        if (++it > kWideSpinLimit) {
+            atomicOr(status, kStatusWideTimeout);
+            return 0ull;
+        }
+        if (it > 16) __nanosleep(64);
+    }
+    return v;
+}
+
+// A tile of small ops: a run of ops of one phase, or whole phases one after
+// another.  Out of line, so that its registers are not the large ops'.
+__device__ __noinline__ void wide_small_tile(WideShared& s, const uint4* ip, uint32_t tile, float2* arenas,
+                                             const uint4* blobs, const float2* table) {
+    __builtin_assume(__isShared(&s));
+    const uint32_t tid = threadIdx.x;
+    const uint4 i0 = __ldg(ip), i1 = __ldg(ip + 1), i2 = __ldg(ip + 2);
+    float2* arena = arenas + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
+    const char* plan = reinterpret_cast<const char*>(blobs) + ((uint64_t)i0.z | (uint64_t)i0.w << 32);
+    const DevOp* ops = reinterpret_cast<const DevOp*>(plan);
+    const DevIn* ins = reinterpret_cast<const DevIn*>(plan + i1.x);
+    const uint4* phases = reinterpret_cast<const uint4*>(plan) - i1.w;
+    const bool chain = (__ldg(&reinterpret_cast<const WideItem*>(ip)->kind_net) & 3u) == kWideChain;
+    const uint32_t e0 = i1.w + tile * i2.y;   // elements of the phase
+    for (uint32_t p = chain ? i1.y : 0u; p < (chain ? i1.z : 1u); ++p) {
+        uint32_t lo = i1.y, hi = i1.z, g = e0 + tid, g_end = min(e0 + i2.y, i2.x);
+        if (chain) {
+            const uint4 ph = __ldg(phases + p);   // first op, ops, elements
+            lo = ph.x;
+            hi = ph.x + ph.y;
+            g = tid;
+            g_end = ph.z;
+        }
+        const bool staged = hi - lo <= kWideSmemOps;
+        if (staged && hi - lo > 1u)
+            for (uint32_t o = tid; o < hi - lo; o += kWideThreads) s.op_first[o] = __ldg(&ops[lo + o].elem_begin);
+        __syncthreads();   // (and the phase before is written)
+        for (; g < g_end; g += kWideSmallTile)
+            wide_small(ops, lo, hi, g, g_end, staged ? s.op_first : nullptr, ins, table, arena);
+        if (chain) __syncthreads();
+    }
+}
+
+// Arena reads are plain loads: the queue's acquire and the barrier after it
+// order them after the other CTAs' writes, and operands that lack some of a
+// tile's element bits (an operand holds about half of them) are reused from
+// L1.  What bounds the kernel is the latency of a tile's dependent steps
+// (ticket, place, item, operand descriptors, then one round of loads per
+// operand), hence four small CTAs per SM, and the next ticket taken ahead
+// while more tiles are ready than CTAs run.  Energies of 3-regular N=256
+// p=4 and Erdos-Renyi N=400 p=3 graphs: 1030 and 1490 us with whole-GPU
+// steps (every tile waited for every network's previous phase, and thread
+// by thread for its own lookups), 432 and 541 us so.  Measured and not
+// kept: three CTAs per SM with the next operand's loads in flight (480 and
+// 635 us), the finishing CTA going on with its network's next phase while
+// it holds a ticket (482 and 635 us: the ticket's tile waits for it).
+__global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm) qtb_wide_kernel(const WideArgs w, const RunArgs a) {
+    __shared__ WideShared s;
+    const uint32_t tid = threadIdx.x;
+    uint32_t ticket = 0;   // thread 0's
+    if (tid == 0) ticket = atomicAdd(w.counters, 1u);
     for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(w.counters, 1u);
-        __syncthreads();
-        const uint32_t t = s_tile;
-        if (t > w.n_tiles) break;
-        uint32_t s = w.n_steps;   // the result tile follows the last step
-        if (t < w.n_tiles) {
-            uint32_t lo = 0, hi = w.n_steps - 1u;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1u) >> 1;
-                if (__ldg(&w.steps[mid].tile_begin) <= t) lo = mid;
-                else hi = mid - 1u;
-            }
-            s = lo;
-        }
-        if (threadIdx.x == 0) {
-            s_ok = 1;
-            if (s > 0 && !wait_counter(w.counters + s, __ldg(&w.steps[s - 1].n_tiles), kWideSpinLimit,
-                                       a.status, kStatusWideTimeout))
-                s_ok = 0;
+        if (tid == 0) {
+            s.place = wide_place(w, ticket, a.status);
             __threadfence();
         }
         __syncthreads();
-        if (!s_ok) return;
-        if (t == w.n_tiles) {
-            // every step is done: the wave's terms, then the run's energy if
-            // this wave finished the run's last networks
-            for (uint32_t n = threadIdx.x; n < w.n_nets; n += blockDim.x) {
-                const WideNet wn = w.nets[n];
-                const DevNetRun net = *wn.run;
-                const float2* arena = w.arenas + wn.arena_off;
-                *wn.term = (net.result_src & kSrcTable) ? __ldg(a.gtable + (net.result_src & ~kSrcTable))
-                                                        : __ldcg(arena + net.result_src);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                s_last = 0;
-                if (a.energy) {
-                    __threadfence();
-                    s_last = atomicAdd(a.done, w.n_nets) == a.total_jobs - w.n_nets;
+        const unsigned long long place = s.place;
+        if (place == 0ull) return;
+        // where more places are filled than CTAs run, the next ticket's is:
+        // taking it now hides the ticket's round trip and keeps nothing waiting
+        uint32_t next = 0xffffffffu;
+        if (tid == 0 && ticket + gridDim.x < w.n_ready + __ldcg(w.counters + 1)) next = atomicAdd(w.counters, 1u);
+        const uint4* ip = reinterpret_cast<const uint4*>(w.items + ((uint32_t)(place >> 32) - 1u));
+        const uint32_t kind = __ldg(&reinterpret_cast<const WideItem*>(ip)->kind_net) & 3u;
+        if (kind == kWideOp) {
+            const uint4 i0 = __ldg(ip), i1 = __ldg(ip + 1), i2 = __ldg(ip + 2);
+            float2* arena = w.arenas + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
+            const char* plan = reinterpret_cast<const char*>(a.blobs) + ((uint64_t)i0.z | (uint64_t)i0.w << 32);
+            const uint32_t e0 = (uint32_t)place * i2.y;   // elements of the op
+            // in groups of chunks; what a group needs is read from the item
+            // again, so that little stays in registers while chunks run
+            for (uint32_t c0 = 0;; c0 += kWideGroup) {
+                const uint32_t k = (i1.y >> 8) & 0xffu;
+                const bool sum = i1.y >> 16;
+                const uint32_t n = min((min(e0 + i2.y, i2.x) - e0) / kWideChunk - c0, kWideGroup);
+                wide_prepare(s, reinterpret_cast<const DevIn*>(plan), k, i1.y & 0xffu, sum, e0 + c0 * kWideChunk, n,
+                             c0 == 0u, w.vec, a.gtable, arena);
+                __syncthreads();
+                if (c0 == 0u)
+                    for (uint32_t q = 0; q < k; ++q) s.off[q][tid] = s.lane[q][tid & 31u] + s.warp[q][tid >> 5];
+                const bool last_group = c0 + kWideGroup >= (min(e0 + i2.y, i2.x) - e0) / kWideChunk;
+                float2* out = arena + i1.x + e0 + c0 * kWideChunk + 2u * tid;
+                for (uint32_t c = 0; c < n; ++c, out += kWideChunk) {
+                    float2 p0[4], p1[4];
+                    wide_load(s.ptr[0][c] + s.off[0][tid], s.meta[0], p0, p1);
+#pragma unroll 1
+                    for (uint32_t q = 1; q < k; ++q) {
+                        float2 x0[4], x1[4];
+                        wide_load(s.ptr[q][c] + s.off[q][tid], s.meta[q], x0, x1);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            p0[e] = cmul(p0[e], x0[e]);
+                            p1[e] = cmul(p1[e], x1[e]);
+                        }
+                    }
+                    if (sum)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) p0[e] = make_float2(p0[e].x + p1[e].x, p0[e].y + p1[e].y);
+                    if (w.vec) {
+                        reinterpret_cast<float4*>(out)[0] = make_float4(p0[0].x, p0[0].y, p0[1].x, p0[1].y);
+                        reinterpret_cast<float4*>(out + kWideChunk / 2)[0] =
+                            make_float4(p0[2].x, p0[2].y, p0[3].x, p0[3].y);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) out[(e & 1) + (e >> 1) * (kWideChunk / 2)] = p0[e];
+                    }
                 }
+                if (last_group) break;
+                __syncthreads();
             }
-            __syncthreads();
-            if (s_last) {
+        } else {
+            wide_small_tile(s, ip, (uint32_t)place, w.arenas, a.blobs, a.gtable);
+        }
+        __syncthreads();
+        // the CTA that finishes a phase queues the network's next one; after
+        // the last phase it writes the network's term, and the CTA that
+        // finishes the run's last network its energy
+        const uint4 i3 = __ldg(ip + 3);   // next phase: first item, items, tiles; kind and network
+        if (tid == 0) {
+            const uint2 count = __ldg(reinterpret_cast<const uint2*>(ip + 2) + 1);   // done, need
+            s.last = 0;
+            __threadfence();
+            s.finished = atomicAdd(w.counters + count.x, 1u) == count.y - 1u;
+            if (s.finished) {
                 __threadfence();
-                reduce_energy(a.terms, a.total_jobs, a.energy_groups, a.energy);
-                if (threadIdx.x == 0) *a.done = 0u;
-            }
-            break;
-        }
-        const WideStep st = w.steps[s];
-        const uint32_t e0 = (t - st.tile_begin) * st.tile_elems;
-        const uint32_t e1 = min(e0 + st.tile_elems, st.total_elems);
-        // per-thread cache of the current segment and op
-        uint32_t seg_lo = 1u, seg_hi = 0u, op_lo = 1u, op_hi = 0u, ph_total = 0u;
-        const unsigned char* blob = nullptr;
-        const DevIn* ins = nullptr;
-        const DevOp* ops = nullptr;
-        const uint16_t* chunk = nullptr;
-        float2* arena = nullptr;
-        DevOp op{};
-        uint32_t op_first = 0, op_last = 0;
-        const uint32_t bd = blockDim.x;
-        for (uint32_t g = e0 + threadIdx.x; g < e1;) {
-            if (g < seg_lo || g >= seg_hi) {
-                uint32_t lo = st.seg_begin, hi = st.seg_begin + st.n_segs - 1u;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi + 1u) >> 1;
-                    if (__ldg(&w.segs[mid].elem_begin) <= g) lo = mid;
-                    else hi = mid - 1u;
+                if (!(i3.w & 4u)) {
+                    s.first_place = atomicAdd(w.counters + 1, i3.z);
+                } else {
+                    const WideNet wn = w.nets[i3.w >> 3];
+                    const uint32_t src = wn.run->result_src;
+                    *wn.term = (src & kSrcTable) ? a.gtable[src & ~kSrcTable] : __ldcg(w.arenas + wn.arena_off + src);
+                    if (a.energy) {
+                        __threadfence();
+                        s.last = atomicAdd(a.done, 1u) == a.total_jobs - 1u;
+                    }
                 }
-                const WideSeg sg = w.segs[lo];
-                seg_lo = sg.elem_begin;
-                seg_hi = lo + 1u < st.seg_begin + st.n_segs ? __ldg(&w.segs[lo + 1u].elem_begin) : st.total_elems;
-                const WideNet wn = w.nets[sg.net];
-                const DevNetRun net = *wn.run;
-                blob = reinterpret_cast<const unsigned char*>(a.blobs + net.blob_off16);
-                const DevPhase ph = reinterpret_cast<const DevPhase*>(blob)[s];
-                ph_total = ph.total_elems;
-                ops = reinterpret_cast<const DevOp*>(blob + net.n_phases * sizeof(DevPhase));
-                ins = reinterpret_cast<const DevIn*>(blob + net.ins_off);
-                chunk = ph.chunk_off ? reinterpret_cast<const uint16_t*>(blob + ph.chunk_off) : nullptr;
-                arena = w.arenas + wn.arena_off;
-                op_first = ph.op_first;
-                op_last = ph.op_first + ph.op_count - 1u;
-                op_lo = 1u;
-                op_hi = 0u;
             }
-            const uint32_t l = g - seg_lo;
-            if (l >= ph_total) {   // padding between segments
-                g += bd;
-                continue;
-            }
-            if (l < op_lo || l >= op_hi) {
-                const uint32_t oi = chunk ? __ldg(chunk + l / kChunkElems) : search_op<true>(ops, op_first, op_last, l);
-                op = ldg_op(ops + oi);
-                find_op(l, oi, op, [&](uint32_t i) { return ldg_op(ops + min(i, op_last)); });
-                op_lo = op.elem_begin;
-                op_hi = op.elem_begin + (1u << (op.u - op.sum));
-            }
-            // 2^kBatchLog elements of the same op that differ only in the bits
-            // from bit 8 up of the op index (the common case in wide phases:
-            // tiles, segments and ops start at multiples of kWideMinTile)
-            const uint32_t j = l - op.elem_begin;
-            if (bd == 256u && (j & kBatchBits) == 0u && g + (kB - 1) * bd < min(e1, seg_hi) &&
-                l + (kB - 1) * bd < op_hi) {
-                compute_elements_wide<kBatchLog>(op, j, ins, a.gtable, arena);
-                g += kB * bd;
-            } else {
-                compute_element_wide(op, j, ins, a.gtable, arena);
-                g += bd;
-            }
+            ticket = next != 0xffffffffu ? next : atomicAdd(w.counters, 1u);
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (s.finished && !(i3.w & 4u)) {
+            unsigned long long* q = w.queue + s.first_place;
+            for (uint32_t i = 0; i < i3.y; ++i) {
+                const uint4 n1 = __ldg(reinterpret_cast<const uint4*>(w.items + i3.x + i) + 1);
+                const uint4 n2 = __ldg(reinterpret_cast<const uint4*>(w.items + i3.x + i) + 2);
+                const bool one = n2.y == 0u;   // a chain
+                const uint32_t tiles = one ? 1u : (n2.x - n1.w + n2.y - 1u) / n2.y;
+                for (uint32_t t = tid; t < tiles; t += kWideThreads)
+                    st_release64(q + t, (unsigned long long)(i3.x + i + 1u) << 32 | t);
+                q += tiles;
+            }
+        }
+        if (s.last) {
             __threadfence();
-            atomicAdd(w.counters + 1 + s, 1u);
+            reduce_energy_call(a.terms, a.total_jobs, a.energy_groups, a.energy);
+            if (tid == 0) *a.done = 0u;   // ready for the next run
         }
     }
 }
@@ -1396,7 +1619,7 @@ __global__ void __launch_bounds__(kClusterThreads) qtb_cluster_kernel(const Clus
             const uint32_t size = 1u << (op.u - op.sum);
             if (size >= kClusterChunk && base + kClusterChunk <= total) {
                 // the whole chunk lies in this op (ops start at multiples of their size)
-                compute_elements_wide<kWideBatchLog>(op, base + t - op.elem_begin, ins, a.gtable, arena);
+                compute_elements_wide(op, base + t - op.elem_begin, ins, a.gtable, arena);
             } else {
                 uint32_t op_hi = op.elem_begin + size;
 #pragma unroll 1
@@ -1496,8 +1719,8 @@ static CommonImage common_image(const qtb_plan* plan) {
 
 // One wave of wide networks: its tables live in RunCache::wide_buf.
 struct WideWave {
-    size_t nets_off, steps_off, segs_off, counters_off;   // bytes into wide_buf
-    uint32_t n_nets, n_steps, n_tiles;
+    size_t nets_off, items_off, ready_off, queue_off, counters_off;   // bytes into wide_buf
+    uint32_t n_nets, n_tiles, n_ready;
     int grid;
 };
 
@@ -1515,9 +1738,8 @@ struct RunCache {
     std::vector<LaunchClass> h12classes;  // the same with the 96-thread lean queue (12 CTAs per SM)
     std::vector<LaunchClass> wclasses;  // warp schedule: large networks as classes + warp queue
     std::vector<WideWave> waves;        // wide networks (both schedules), run one after another
-    int wide_batch_log = kWideBatchLog; // wave kernel variant: 2^this elements per thread in flight
     void* wide_buf = nullptr;
-    size_t counters_bytes = 0;          // counters of all waves, zeroed before a run
+    size_t zeroed_off = 0, zeroed_bytes = 0;   // queues and counters of all waves, zeroed before a run
     size_t scratch_elems = 0;           // arenas of the largest wave, then the cluster arenas
     void* cl_jobs = nullptr;            // ClusterJob per network of moderate size (K5)
     int n_cl = 0;
@@ -1813,15 +2035,123 @@ static size_t net_need(const DevNetRun& r, size_t fixed, bool records) {
 
 // Wide waves of a run: the networks too large for shared memory, largest
 // arena first, packed into waves whose arenas fit kWideWaveBytes (a larger
-// network forms a wave of its own).  Per wave: networks, steps (one per
-// phase index, its segments the wave networks that have that phase) and
-// tiles of kWideTileElems elements; one device buffer holds all tables.
+// network forms a wave of its own); one device buffer holds all their
+// tables.
 constexpr size_t kWideWaveBytes = size_t(1) << 30;
+
+// The items of one wave's networks `members` (see WideItem), the places of
+// the queue that are filled from the start (the first phase of every
+// network), the tiles of the wave and its counters.  `slots`: resident CTAs,
+// which the tiles of large ops are sized for.
+struct WideTables {
+    std::vector<WideItem> items;
+    std::vector<unsigned long long> ready;
+    uint32_t n_tiles = 0, n_counters = 2;
+};
+
+static uint32_t item_tiles(const WideItem& it) {
+    return it.tile_elems ? (it.elem_end - it.elem_begin + it.tile_elems - 1) / it.tile_elems : 1u;
+}
+
+static WideTables wave_tables(const qtb_plan* plan, const std::vector<int32_t>& members,
+                              const std::vector<uint64_t>& arena_off, uint64_t slots) {
+    auto large = [](const DevOp& op) { return op.k <= kWideMaxK && (1u << (op.u - op.sum)) >= kWideChunk; };
+    // elements of large ops per phase index, over all networks
+    std::vector<uint64_t> op_elems;
+    for (int32_t m : members) {
+        const Network& n = plan->nets[m];
+        op_elems.resize(std::max(op_elems.size(), n.phases.size()), 0);
+        for (size_t ph = 0; ph < n.phases.size(); ++ph)
+            for (uint32_t o = n.phases[ph].op_first; o < n.phases[ph].op_first + n.phases[ph].op_count; ++o)
+                if (large(n.ops[o])) op_elems[ph] += 1ull << (n.ops[o].u - n.ops[o].sum);
+    }
+    WideTables out;
+    for (size_t k = 0; k < members.size(); ++k) {
+        const Network& n = plan->nets[members[k]];
+        const DevNetRun& run = plan->druns[members[k]];
+        const uint32_t np = (uint32_t)n.phases.size();
+        const uint64_t blob = 16 * (uint64_t)run.blob_off16;
+        WideItem base{};
+        base.arena_off = arena_off[k];
+        base.plan_off = blob + np * sizeof(DevPhase);
+        base.a = run.ins_off - np * (uint32_t)sizeof(DevPhase);
+        base.kind_net = (uint32_t)k << 3;
+        size_t prev_begin = 0, prev_end = 0;   // the items of the phase before
+        uint32_t ph = 0;
+        do {
+            uint32_t end = ph;
+            while (end < np && n.phases[end].total_elems <= kWideChainElems) ++end;
+            const size_t first = out.items.size();
+            base.done = out.n_counters++;
+            if (end > ph || np == 0) {
+                // np == 0: the result is a gate-table scalar, and an empty chain writes the term
+                WideItem it = base;
+                it.kind_net |= kWideChain;
+                it.begin = ph;
+                it.end = end;
+                it.elem_begin = np;
+                out.items.push_back(it);
+            } else {
+                end = ph + 1;
+                const DevPhase& p = n.phases[ph];
+                const uint32_t o_end = p.op_first + p.op_count;
+                // about one tile per resident CTA over the networks' phases
+                // of this index: larger tiles spread a tile's set-up over
+                // more chunks, and networks at other phases fill the rest
+                const uint32_t chunks = (uint32_t)std::max<uint64_t>(
+                    1, std::min<uint64_t>(kWideMaxTileChunks, op_elems[ph] / (slots * kWideChunk)));
+                for (uint32_t o = p.op_first; o < o_end;) {
+                    uint32_t q = o + 1;
+                    WideItem it = base;
+                    if (large(n.ops[o])) {
+                        const DevOp& op = n.ops[o];
+                        it.kind_net |= kWideOp;
+                        it.plan_off = blob + run.ins_off + op.in_begin * sizeof(DevIn);
+                        it.a = op.dst;
+                        it.begin = (uint32_t)(op.u - op.sum) | (uint32_t)op.k << 8 | (uint32_t)op.sum << 16;
+                        it.elem_end = 1u << (op.u - op.sum);
+                        it.tile_elems = chunks * kWideChunk;
+                    } else {
+                        while (q < o_end && !large(n.ops[q])) ++q;
+                        it.kind_net |= kWideSmall;
+                        it.begin = o;
+                        it.end = q;
+                        it.elem_begin = n.ops[o].elem_begin;
+                        it.elem_end = q < o_end ? n.ops[q].elem_begin : p.total_elems;
+                        it.tile_elems = kWideSmallTile;
+                    }
+                    out.items.push_back(it);
+                    o = q;
+                }
+            }
+            uint32_t tiles = 0;
+            for (size_t i = first; i < out.items.size(); ++i) tiles += item_tiles(out.items[i]);
+            for (size_t i = first; i < out.items.size(); ++i) {
+                out.items[i].need = tiles;
+                if (end == np) out.items[i].kind_net |= 4u;
+            }
+            for (size_t i = prev_begin; i < prev_end; ++i) {
+                out.items[i].next = (uint32_t)first;
+                out.items[i].next_items = (uint32_t)(out.items.size() - first);
+                out.items[i].next_tiles = tiles;
+            }
+            if (prev_end == 0)
+                for (size_t i = first; i < out.items.size(); ++i)
+                    for (uint32_t t = 0; t < item_tiles(out.items[i]); ++t)
+                        out.ready.push_back((unsigned long long)(i + 1) << 32 | t);
+            out.n_tiles += tiles;
+            prev_begin = first;
+            prev_end = out.items.size();
+            ph = end;
+        } while (ph < np);
+    }
+    return out;
+}
 
 static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first, float2* terms,
                        RunCache* rc, bool device) {
     rc->waves.clear();
-    rc->counters_bytes = 0;
+    rc->zeroed_bytes = 0;
     if (wide.empty()) return QTB_OK;
     auto arena_of = [&](int32_t i) { return ((size_t)plan->druns[i].arena_elems + 63) & ~size_t(63); };
     std::stable_sort(wide.begin(), wide.end(), [&](int32_t x, int32_t y) { return arena_of(x) > arena_of(y); });
@@ -1832,22 +2162,14 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
     if (device) {
         QTB_CUDA(cudaGetDevice(&dev));
         QTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qtb_wide_kernel<kWideBatchLog>,
-                                                               kWideThreads, 0));
-        if (plan->wave_ctas_per_sm > 0) per_sm = std::min(per_sm, (int)plan->wave_ctas_per_sm);
+        QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qtb_wide_kernel, kWideThreads, 0));
+        // the setting counts in halves of an SM
+        if (plan->wave_ctas_per_sm > 0)
+            per_sm = std::min(per_sm, (int)std::min(plan->wave_ctas_per_sm, 2) * (kWideCtasPerSm / 2));
     }
-    // QTB_WIDE_TILES_PER_CTA (1..8, default 2) in the environment sets how
-    // many tiles a step is cut into per resident CTA
-    int tiles_per_cta = 2;
-    if (const char* env = std::getenv("QTB_WIDE_TILES_PER_CTA")) {
-        const int v = std::atoi(env);
-        if (v >= 1 && v <= 8) tiles_per_cta = v;
-    }
-    std::vector<WideNet> nets;
-    std::vector<WideStep> steps;
-    std::vector<WideSeg> segs;
-    struct Range { size_t net0, step0, seg0; };
-    std::vector<Range> ranges;
+    const uint64_t slots = (uint64_t)std::max(1, per_sm) * sms;
+    std::vector<std::vector<WideNet>> nets;
+    std::vector<WideTables> tables;
     size_t pos = 0;
     while (pos < wide.size()) {
         // members of this wave
@@ -1858,84 +2180,66 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
         }
         if (elems >= (size_t(1) << 31))
             return fail(QTB_ERR_UNSUPPORTED, "plan_run: network arena of 2^31 elements or more");
-        Range rg{nets.size(), steps.size(), segs.size()};
-        WideWave wv{};
-        wv.n_nets = (uint32_t)(end - pos);
-        uint32_t max_phases = 0;
-        size_t off = 0;
-        for (size_t k = pos; k < end; ++k) {
-            const int32_t i = wide[k];
-            WideNet wn{};
-            wn.run = runs ? runs + i : nullptr;   // null in a size-only build
-            wn.term = terms + (i - first);
-            wn.arena_off = off;
-            off += arena_of(i);
-            nets.push_back(wn);
-            max_phases = std::max(max_phases, plan->druns[i].n_phases);
-        }
-        rc->scratch_elems = std::max(rc->scratch_elems, off);
-        uint32_t tiles = 0;
-        for (uint32_t ph = 0; ph < max_phases; ++ph) {
-            WideStep st{};
-            st.seg_begin = (uint32_t)(segs.size() - rg.seg0);
-            uint32_t total = 0;
-            for (size_t k = pos; k < end; ++k) {
-                const Network& n = plan->nets[wide[k]];
-                if (ph >= n.phases.size()) continue;
-                // segments start at multiples of kWideMinTile, so that with the
-                // ops of a phase sorted widest first the elements a thread
-                // batches differ only in bits 8 and 9 of their op index
-                total = (total + kWideMinTile - 1) & ~(kWideMinTile - 1);
-                segs.push_back(WideSeg{(uint32_t)(k - pos), total});
-                total += n.phases[ph].total_elems;
+        rc->scratch_elems = std::max(rc->scratch_elems, elems);
+        if (device) {
+            const std::vector<int32_t> members(wide.begin() + pos, wide.begin() + end);
+            std::vector<uint64_t> offs;
+            std::vector<WideNet> wn(members.size());
+            size_t off = 0;
+            for (size_t k = 0; k < members.size(); ++k) {
+                wn[k].run = runs + members[k];
+                wn[k].term = terms + (members[k] - first);
+                wn[k].arena_off = off;
+                offs.push_back(off);
+                off += arena_of(members[k]);
             }
-            st.n_segs = (uint32_t)(segs.size() - rg.seg0) - st.seg_begin;
-            st.total_elems = total;
-            st.tile_begin = tiles;
-            // about `tiles_per_cta` tiles per resident CTA, within
-            // [kWideMinTile, kWideMaxTile]
-            const uint32_t target = total / (uint32_t)(tiles_per_cta * std::max(1, per_sm) * sms) + 1;
-            st.tile_elems = std::min(kWideMaxTile, ((target + kWideMinTile - 1) / kWideMinTile) * kWideMinTile);
-            st.n_tiles = std::max(1u, (total + st.tile_elems - 1) / st.tile_elems);
-            tiles += st.n_tiles;
-            steps.push_back(st);
+            WideTables tb = wave_tables(plan, members, offs, slots);
+            WideWave wv{};
+            wv.n_nets = (uint32_t)members.size();
+            wv.n_tiles = tb.n_tiles;
+            wv.n_ready = (uint32_t)tb.ready.size();
+            wv.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(wv.n_tiles, slots));
+            rc->waves.push_back(wv);
+            nets.push_back(std::move(wn));
+            tables.push_back(std::move(tb));
+        } else {
+            rc->waves.push_back(WideWave{});
         }
-        wv.n_steps = max_phases;
-        wv.n_tiles = tiles;
-        wv.grid = std::max(1, std::min<int>((int)tiles + 1, std::max(1, per_sm) * sms));
-        rc->waves.push_back(wv);
-        ranges.push_back(rg);
         pos = end;
     }
-    // device image: per wave [nets][steps][segs][counters], 256-byte aligned
+    if (!device) return QTB_OK;   // sizes only (qtb_plan_scratch_bytes)
+    // device buffer: per wave [nets][items][ready], 256-byte aligned, then
+    // per wave [queue][counters], which are zeroed before a run
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     size_t bytes = 0;
     for (size_t v = 0; v < rc->waves.size(); ++v) {
         WideWave& wv = rc->waves[v];
-        const size_t n_segs = (v + 1 < ranges.size() ? ranges[v + 1].seg0 : segs.size()) - ranges[v].seg0;
         wv.nets_off = bytes;
-        bytes = align(bytes + wv.n_nets * sizeof(WideNet));
-        wv.steps_off = bytes;
-        bytes = align(bytes + wv.n_steps * sizeof(WideStep));
-        wv.segs_off = bytes;
-        bytes = align(bytes + n_segs * sizeof(WideSeg));
+        bytes = align(bytes + nets[v].size() * sizeof(WideNet));
+        wv.items_off = bytes;
+        bytes = align(bytes + tables[v].items.size() * sizeof(WideItem));
+        wv.ready_off = bytes;
+        bytes = align(bytes + tables[v].ready.size() * sizeof(unsigned long long));
     }
-    const size_t counters0 = bytes;
-    for (WideWave& wv : rc->waves) {
+    const size_t zeroed = bytes;
+    for (size_t v = 0; v < rc->waves.size(); ++v) {
+        WideWave& wv = rc->waves[v];
+        wv.queue_off = bytes;
+        bytes += (size_t)(wv.n_tiles - wv.n_ready) * sizeof(unsigned long long);
         wv.counters_off = bytes;
-        bytes += (1 + (size_t)wv.n_steps) * sizeof(unsigned int);
+        bytes += ((size_t)tables[v].n_counters * sizeof(unsigned int) + 7) & ~size_t(7);
     }
-    rc->counters_bytes = bytes - counters0;
-    if (!device) return QTB_OK;   // sizes only (qtb_plan_scratch_bytes)
-    std::vector<uint8_t> image(align(bytes), 0);
+    rc->zeroed_off = zeroed;
+    rc->zeroed_bytes = bytes - zeroed;
+    std::vector<uint8_t> image(zeroed, 0);
     for (size_t v = 0; v < rc->waves.size(); ++v) {
         const WideWave& wv = rc->waves[v];
-        const size_t n_segs = (v + 1 < ranges.size() ? ranges[v + 1].seg0 : segs.size()) - ranges[v].seg0;
-        std::memcpy(image.data() + wv.nets_off, nets.data() + ranges[v].net0, wv.n_nets * sizeof(WideNet));
-        std::memcpy(image.data() + wv.steps_off, steps.data() + ranges[v].step0, wv.n_steps * sizeof(WideStep));
-        std::memcpy(image.data() + wv.segs_off, segs.data() + ranges[v].seg0, n_segs * sizeof(WideSeg));
+        std::memcpy(image.data() + wv.nets_off, nets[v].data(), nets[v].size() * sizeof(WideNet));
+        std::memcpy(image.data() + wv.items_off, tables[v].items.data(), tables[v].items.size() * sizeof(WideItem));
+        std::memcpy(image.data() + wv.ready_off, tables[v].ready.data(),
+                    tables[v].ready.size() * sizeof(unsigned long long));
     }
-    QTB_CUDA(cudaMalloc(&rc->wide_buf, image.size()));
+    QTB_CUDA(cudaMalloc(&rc->wide_buf, bytes));
     QTB_CUDA(cudaMemcpy(rc->wide_buf, image.data(), image.size(), cudaMemcpyHostToDevice));
     return QTB_OK;
 }
@@ -2134,12 +2438,6 @@ static int build_run(qtb_plan* plan, int32_t first, int32_t count, float2* terms
     if (const char* env = std::getenv("QTB_CLUSTER_MAX_ELEMS")) cl_max = std::strtoull(env, nullptr, 10);
     for (int32_t i : members[kSmemClasses])
         (plan->druns[i].arena_elems <= cl_max ? cl_nets : wave_nets).push_back(i);
-    // QTB_WIDE_BATCH=2 or 3 in the environment fixes the wave kernel variant
-    // (2^this elements per thread in flight) instead of the autotuner
-    if (const char* env = std::getenv("QTB_WIDE_BATCH")) {
-        const int v = std::atoi(env);
-        if (v == 2 || v == 3) rc->wide_batch_log = v;
-    }
     // QTB_CLUSTER_CTAS (2, 4, 8 or 16) sets the CTAs per cluster
     rc->cl_ctas = kClusterCtas;
     if (const char* env = std::getenv("QTB_CLUSTER_CTAS")) {
@@ -2335,19 +2633,19 @@ static int launch_waves(const RunCache* rc, const RunArgs& base, void* scratch_d
     }
     if (rc->waves.empty()) return QTB_OK;
     char* buf = static_cast<char*>(rc->wide_buf);
-    QTB_CUDA(cudaMemsetAsync(buf + rc->waves[0].counters_off, 0, rc->counters_bytes, st));
+    QTB_CUDA(cudaMemsetAsync(buf + rc->zeroed_off, 0, rc->zeroed_bytes, st));
     for (const WideWave& wv : rc->waves) {
         WideArgs w{};
         w.nets = reinterpret_cast<const WideNet*>(buf + wv.nets_off);
-        w.steps = reinterpret_cast<const WideStep*>(buf + wv.steps_off);
-        w.segs = reinterpret_cast<const WideSeg*>(buf + wv.segs_off);
+        w.items = reinterpret_cast<const WideItem*>(buf + wv.items_off);
+        w.queue = reinterpret_cast<unsigned long long*>(buf + wv.queue_off);
+        w.ready = reinterpret_cast<const unsigned long long*>(buf + wv.ready_off);
         w.counters = reinterpret_cast<unsigned int*>(buf + wv.counters_off);
         w.arenas = static_cast<float2*>(scratch_dev);
-        w.n_nets = wv.n_nets;
-        w.n_steps = wv.n_steps;
         w.n_tiles = wv.n_tiles;
-        if (rc->wide_batch_log == 2) qtb_wide_kernel<2><<<wv.grid, kWideThreads, 0, st>>>(w, base);
-        else qtb_wide_kernel<kWideBatchLog><<<wv.grid, kWideThreads, 0, st>>>(w, base);
+        w.n_ready = wv.n_ready;
+        w.vec = reinterpret_cast<uintptr_t>(scratch_dev) % 16 == 0;
+        qtb_wide_kernel<<<wv.grid, kWideThreads, 0, st>>>(w, base);
         QTB_CUDA(cudaGetLastError());
     }
     return QTB_OK;
@@ -2355,7 +2653,9 @@ static int launch_waves(const RunCache* rc, const RunArgs& base, void* scratch_d
 
 // Launch a schedule on st: a persistent class needs its queue zeroed first
 // (a memset node when captured); several classes, and the wide waves, run
-// concurrently on forked streams joined back into st.
+// concurrently on forked streams joined back into st.  The waves come last:
+// a wave's CTAs stay for its whole run, so the classes take their SMs first
+// and the wave grows into them.
 static int launch_schedule(qtb_plan_device* s, const RunCache* rc,
                            const std::vector<LaunchClass>& sched, const RunArgs& base,
                            void* scratch_dev, cudaStream_t st, bool with_waves = true) {
@@ -2366,15 +2666,6 @@ static int launch_schedule(qtb_plan_device* s, const RunCache* rc,
     const bool waves = with_waves && (!rc->waves.empty() || rc->n_cl > 0);
     const bool forked = sched.size() + (waves ? 1 : 0) > 1;
     if (forked) QTB_CUDA(cudaEventRecord(s->fork, st));
-    if (waves) {
-        cudaStream_t ws = forked ? s->aux[kMaxClasses - 1] : st;
-        if (forked) QTB_CUDA(cudaStreamWaitEvent(ws, s->fork, 0));
-        if ((r = launch_waves(rc, base, scratch_dev, ws))) return r;
-        if (forked) {
-            QTB_CUDA(cudaEventRecord(s->join[kMaxClasses - 1], ws));
-            QTB_CUDA(cudaStreamWaitEvent(st, s->join[kMaxClasses - 1], 0));
-        }
-    }
     for (size_t c = 0; c < sched.size(); ++c) {
         const LaunchClass& lc = sched[c];
         cudaStream_t cs = forked ? s->aux[c] : st;
@@ -2393,6 +2684,15 @@ static int launch_schedule(qtb_plan_device* s, const RunCache* rc,
             QTB_CUDA(cudaStreamWaitEvent(st, s->join[c], 0));
         }
     }
+    if (waves) {
+        cudaStream_t ws = forked ? s->aux[kMaxClasses - 1] : st;
+        if (forked) QTB_CUDA(cudaStreamWaitEvent(ws, s->fork, 0));
+        if ((r = launch_waves(rc, base, scratch_dev, ws))) return r;
+        if (forked) {
+            QTB_CUDA(cudaEventRecord(s->join[kMaxClasses - 1], ws));
+            QTB_CUDA(cudaStreamWaitEvent(st, s->join[kMaxClasses - 1], 0));
+        }
+    }
     return QTB_OK;
 }
 
@@ -2404,6 +2704,15 @@ static int launch_schedule(qtb_plan_device* s, const RunCache* rc,
 static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, void* scratch_dev,
                         cudaStream_t st) {
     static const int kCandidates[] = {64, 128, 256, 512, 1024};
+    if (!rc->waves.empty()) {
+        // a wave outlasts the other networks' launches, which run in its
+        // shadow; timed beside it they differ by less than the launch order
+        // does (a tuned choice took between 456 and 645 us on N=256 p=4,
+        // the classes with their default blocks 432 us on every run)
+        rc->schedule = kSchedClasses;
+        rc->tuned = true;
+        return QTB_OK;
+    }
     cudaEvent_t e0, e1;
     QTB_CUDA(cudaEventCreate(&e0));
     QTB_CUDA(cudaEventCreate(&e1));
@@ -2587,21 +2896,6 @@ static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, v
                      : rc->schedule == kSchedHybrid   ? "hybrid"
                      : rc->schedule == kSchedPersistent ? "persistent"
                                                       : "classes");
-    }
-    // the wave kernel variant (8 or 4 elements per thread in flight), timed
-    // with the chosen schedule unless QTB_WIDE_BATCH fixes it
-    if (!rc->waves.empty() && !std::getenv("QTB_WIDE_BATCH")) {
-        float wave_ms[2] = {1e30f, 1e30f};
-        for (int v = 0; v < 2; ++v) {
-            rc->wide_batch_log = v == 0 ? (int)kWideBatchLog : 2;
-            if ((r = time_it([&] { return launch_schedule(s, rc, schedule_of(rc), a, scratch_dev, st); },
-                             &wave_ms[v])))
-                return r;
-        }
-        rc->wide_batch_log = wave_ms[1] < wave_ms[0] ? 2 : (int)kWideBatchLog;
-        if (log)
-            std::fprintf(stderr, "qtb autotune: waves with 8 elements per thread %.1f us, 4 elements %.1f us\n",
-                         1e3 * wave_ms[0], 1e3 * wave_ms[1]);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
