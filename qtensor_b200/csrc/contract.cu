@@ -39,44 +39,186 @@
 #include <algorithm>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
 #include "plan.h"
 
 namespace qtb {
 
 // ----------------------------------------------------------------- CUDA cores
-// c[n,m,k] = a[n,m] * b[n,k], one element per thread (grid-stride).
-__global__ void qtb_outer_kernel(const float2* __restrict__ a, const float2* __restrict__ b,
-                                 float2* __restrict__ c, uint64_t n, uint64_t m, uint64_t k) {
-    const uint64_t total = n * m * k;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t kk = i % k, mm = (i / k) % m, nn = i / (k * m);
-        const float2 x = a[nn * m + mm], y = b[nn * k + kk];
-        c[i] = make_float2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
+// The outputs of both kernels below are [F][M][N]; a thread takes a block of
+// kRows rows (m) x 1 or 2 columns (n), then the block one grid width further.
+// A block's index (f, row block, column block) is divided out once and every
+// step adds the grid width in the same mixed radix, so that the loop has no
+// division: two 64-bit divisions per output made the kernels issue-bound
+// (1.8 TB/s of 6.5 for the outer product, 1.2 TB/s for K = 2).  Rows in a
+// block share the load of their b, and with kPairs (N even, 16-byte aligned
+// pointers) two columns load and store 16 bytes.  256 x 256 x 256 outer
+// product: 73.7 -> 24.6 us; K = 2, F = 64, M = N = 512: 116 -> 33 us (134 MB
+// written; a memset of it takes 20.6 us).
+// I: 32-bit indices, or 64-bit where a dimension needs them.
+template <typename I>
+struct FlatIndex {
+    uint64_t f;
+    I m, n;
+};
+
+template <typename I>
+struct FlatShape {
+    uint64_t blocks;     // F x row blocks x column blocks
+    I M, N;
+    I rows, cols;        // row and column blocks
+    FlatIndex<I> step;   // the grid width
+};
+
+template <typename I>
+__device__ __forceinline__ FlatIndex<I> flat_start(uint64_t i, const FlatShape<I>& s) {
+    const uint64_t row = i / s.cols;
+    return FlatIndex<I>{row / s.rows, (I)(row % s.rows), (I)(i % s.cols)};
+}
+
+template <typename I>
+__device__ __forceinline__ void flat_step(FlatIndex<I>& x, const FlatShape<I>& s) {
+    x.n += s.step.n;
+    x.m += s.step.m;
+    x.f += s.step.f;
+    if (x.n >= s.cols) {
+        x.n -= s.cols;
+        ++x.m;
+    }
+    if (x.m >= s.rows) {
+        x.m -= s.rows;
+        ++x.f;
     }
 }
 
-// C[f,m,n] = sum_k A[k,f,m] B[k,f,n], one output per thread, FP32 sums
-// over k in order.
-__global__ void qtb_contract_simt_kernel(const float2* __restrict__ A, const float2* __restrict__ B,
-                                         float2* __restrict__ C, uint64_t K, uint64_t F, uint64_t M,
-                                         uint64_t N) {
-    const uint64_t total = F * M * N;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t nn = i % N, mm = (i / N) % M, ff = i / (N * M);
-        float re = 0.f, im = 0.f;
-        for (uint64_t kk = 0; kk < K; ++kk) {
-            const float2 x = A[(kk * F + ff) * M + mm], y = B[(kk * F + ff) * N + nn];
-            re = fmaf(x.x, y.x, re);
-            re = fmaf(-x.y, y.y, re);
-            im = fmaf(x.x, y.y, im);
-            im = fmaf(x.y, y.x, im);
-        }
-        C[i] = make_float2(re, im);
+constexpr int kFlatThreads = 256;
+constexpr int kFlatBlocksPerSm = 4;   // all resident at 64 registers (48 spill: K = 2 41 us; 74 and 8 per SM: 42)
+constexpr int kFlatRows = 4;
+
+template <typename I>
+static FlatShape<I> flat_shape(uint64_t F, uint64_t M, uint64_t N, int block_rows, int block_cols, unsigned* grid) {
+    FlatShape<I> s{};
+    s.M = (I)M;
+    s.N = (I)N;
+    s.rows = (I)((M + block_rows - 1) / block_rows);
+    s.cols = (I)(N / block_cols);
+    s.blocks = F * s.rows * s.cols;
+    *grid = (unsigned)std::min<uint64_t>((s.blocks + kFlatThreads - 1) / kFlatThreads, 148ull * kFlatBlocksPerSm);
+    const uint64_t width = (uint64_t)*grid * kFlatThreads;
+    s.step = FlatIndex<I>{width / s.cols / s.rows, (I)(width / s.cols % s.rows), (I)(width % s.cols)};
+    return s;
+}
+
+// Rows per thread: four where that still leaves every thread of the grid a
+// block and the indices 32 bits, else one (below, the call is launch-bound:
+// 8-9 us with either).
+static int flat_rows(uint64_t outputs, uint64_t M, uint64_t N) {
+    const uint64_t enough = 148ull * kFlatBlocksPerSm * kFlatThreads * kFlatRows;
+    return outputs >= enough && M < (1ull << 30) && N < (1ull << 30) ? kFlatRows : 1;
+}
+
+template <bool kPairs>
+__device__ __forceinline__ void flat_load(const float2* p, float2 (&v)[kPairs ? 2 : 1]) {
+    if constexpr (kPairs) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
+    } else {
+        v[0] = *p;
     }
 }
+
+template <bool kPairs>
+__device__ __forceinline__ void flat_store(float2* p, const float2 (&v)[kPairs ? 2 : 1]) {
+    if constexpr (kPairs) *reinterpret_cast<float4*>(p) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+    else *p = v[0];
+}
+
+// c[f,m,n] = a[f,m] * b[f,n].
+template <int kRows, bool kPairs, typename I>
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_outer_kernel(const float2* __restrict__ a,
+                                                                 const float2* __restrict__ b, float2* __restrict__ c,
+                                                                 const FlatShape<I> s) {
+    constexpr int kCols = kPairs ? 2 : 1;
+    uint64_t i = blockIdx.x * (uint64_t)kFlatThreads + threadIdx.x;
+    if (i >= s.blocks) return;
+    FlatIndex<I> x = flat_start(i, s);
+    for (; i < s.blocks; i += (uint64_t)gridDim.x * kFlatThreads, flat_step(x, s)) {
+        const I m = x.m * kRows, n = x.n * kCols;
+        float2 v[kCols], u[kRows];
+        flat_load<kPairs>(b + x.f * s.N + n, v);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) u[r] = a[x.f * s.M + (kRows == 1 || m + r < s.M ? m + r : m)];
+        float2* out = c + (x.f * s.M + m) * s.N + n;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r, out += s.N) {
+            float2 p[kCols];
+#pragma unroll
+            for (int e = 0; e < kCols; ++e)
+                p[e] = make_float2(fmaf(u[r].x, v[e].x, -(u[r].y * v[e].y)), fmaf(u[r].y, v[e].x, u[r].x * v[e].y));
+            if (kRows == 1 || m + r < s.M) flat_store<kPairs>(out, p);
+        }
+    }
+}
+
+// C[f,m,n] = sum_k A[k,f,m] B[k,f,n], FP32 sums over k in order.  kAhead k
+// values are loaded together, so that a long sum over few outputs waits for
+// memory once per kAhead terms.
+template <int kRows, bool kPairs, int kAhead, typename I>
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_contract_simt_kernel(const float2* __restrict__ A,
+                                                                         const float2* __restrict__ B,
+                                                                         float2* __restrict__ C, uint64_t K,
+                                                                         uint64_t a_stride, uint64_t b_stride,
+                                                                         int* status, const FlatShape<I> s) {
+    constexpr int kCols = kPairs ? 2 : 1;
+    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;   // nothing here can fail
+    uint64_t i = blockIdx.x * (uint64_t)kFlatThreads + threadIdx.x;
+    if (i >= s.blocks) return;
+    FlatIndex<I> x = flat_start(i, s);
+    for (; i < s.blocks; i += (uint64_t)gridDim.x * kFlatThreads, flat_step(x, s)) {
+        const I m = x.m * kRows, n = x.n * kCols;
+        const float2* pa = A + x.f * s.M + m;
+        const float2* pb = B + x.f * s.N + n;
+        float2 sum[kRows][kCols];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+#pragma unroll
+            for (int e = 0; e < kCols; ++e) sum[r][e] = make_float2(0.f, 0.f);
+        auto terms = [&](auto count) {
+            constexpr int kCount = decltype(count)::value;
+            float2 u[kCount][kRows], v[kCount][kCols];
+#pragma unroll
+            for (int k = 0; k < kCount; ++k) {
+                flat_load<kPairs>(pb, v[k]);
+#pragma unroll
+                for (int r = 0; r < kRows; ++r) u[k][r] = pa[kRows == 1 || m + r < s.M ? r : 0];
+                pa += a_stride;
+                pb += b_stride;
+            }
+#pragma unroll
+            for (int k = 0; k < kCount; ++k)
+#pragma unroll
+                for (int r = 0; r < kRows; ++r)
+#pragma unroll
+                    for (int e = 0; e < kCols; ++e) {
+                        sum[r][e].x = fmaf(u[k][r].x, v[k][e].x, sum[r][e].x);
+                        sum[r][e].x = fmaf(-u[k][r].y, v[k][e].y, sum[r][e].x);
+                        sum[r][e].y = fmaf(u[k][r].x, v[k][e].y, sum[r][e].y);
+                        sum[r][e].y = fmaf(u[k][r].y, v[k][e].x, sum[r][e].y);
+                    }
+        };
+        uint64_t k = 0;
+        for (; k + kAhead <= K; k += kAhead) terms(std::integral_constant<int, kAhead>());
+        for (; k < K; ++k) terms(std::integral_constant<int, 1>());
+        float2* out = C + (x.f * s.M + m) * s.N + n;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r, out += s.N)
+            if (kRows == 1 || m + r < s.M) flat_store<kPairs>(out, sum[r]);
+    }
+}
+
+static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 // ----------------------------------------------------------------- tensor cores
 constexpr uint32_t kTcM = 128;                        // output tile rows (A tile rows)
@@ -453,10 +595,20 @@ extern "C" {
 int qtb_contract_outer_c64(const void* a, const void* b, void* c, int64_t n, int64_t m, int64_t k,
                            void* stream) {
     if (!a || !b || !c || n < 1 || m < 1 || k < 1) return fail(QTB_ERR_ARG, "contract_outer: bad arguments");
-    const uint64_t total = (uint64_t)n * m * k;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 148ull * 16);
-    qtb_outer_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float2*>(a), static_cast<const float2*>(b), static_cast<float2*>(c), n, m, k);
+    const float2 *pa = static_cast<const float2*>(a), *pb = static_cast<const float2*>(b);
+    float2* pc = static_cast<float2*>(c);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rows = flat_rows((uint64_t)n * m * k, m, k);
+    const bool pairs = rows > 1 && k % 2 == 0 && aligned16(b) && aligned16(c);
+    unsigned grid = 0;
+    if (rows > 1) {
+        const FlatShape<uint32_t> s = flat_shape<uint32_t>(n, m, k, rows, pairs ? 2 : 1, &grid);
+        if (pairs) qtb_outer_kernel<kFlatRows, true><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
+        else qtb_outer_kernel<kFlatRows, false><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
+    } else {
+        const FlatShape<uint64_t> s = flat_shape<uint64_t>(n, m, k, 1, 1, &grid);
+        qtb_outer_kernel<1, false><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
+    }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_outer launch");
 }
@@ -483,14 +635,25 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
     if (r) return r;
     if (!scratch || scratch_bytes < need)
         return fail(QTB_ERR_ARG, "contract_sum: scratch smaller than qtb_contract_sum_scratch_bytes");
-    cudaError_t e = cudaMemsetAsync(scratch, 0, 16, st);   // status word
-    if (e != cudaSuccess) return cuda_fail_c(e, "contract_sum status reset");
+    int* status = static_cast<int*>(scratch);
+    cudaError_t e = cudaSuccess;
     if (!use_tensor_cores(mode, K, M, N)) {
-        const uint64_t total = (uint64_t)F * M * N;
-        const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 148ull * 16);
-        qtb_contract_simt_kernel<<<blocks, 256, 0, st>>>(static_cast<const float2*>(A),
-                                                         static_cast<const float2*>(B), static_cast<float2*>(C),
-                                                         K, F, M, N);
+        const float2 *pa = static_cast<const float2*>(A), *pb = static_cast<const float2*>(B);
+        float2* pc = static_cast<float2*>(C);
+        const int rows = flat_rows((uint64_t)F * M * N, M, N);
+        const bool pairs = rows > 1 && N % 2 == 0 && aligned16(B) && aligned16(C);   // every k's rows too
+        const uint64_t as = (uint64_t)F * M, bs = (uint64_t)F * N;
+        unsigned grid = 0;
+        if (rows > 1) {
+            const FlatShape<uint32_t> s = flat_shape<uint32_t>(F, M, N, rows, pairs ? 2 : 1, &grid);
+            if (pairs)
+                qtb_contract_simt_kernel<kFlatRows, true, 2><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
+            else
+                qtb_contract_simt_kernel<kFlatRows, false, 2><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
+        } else {
+            const FlatShape<uint64_t> s = flat_shape<uint64_t>(F, M, N, 1, 1, &grid);
+            qtb_contract_simt_kernel<1, false, 8><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
+        }
         e = cudaGetLastError();
         return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
     }
@@ -499,7 +662,8 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
         (uint64_t)F * (Mp / kTcM) * (Kp / kTcStageK) >= (1ull << 31) ||
         (uint64_t)F * (Np / kTcN) * (Kp / kTcStageK) >= (1ull << 31))
         return fail(QTB_ERR_UNSUPPORTED, "contract_sum: shape beyond the tensor-core grid");
-    int* status = static_cast<int*>(scratch);
+    e = cudaMemsetAsync(scratch, 0, 16, st);   // status word
+    if (e != cudaSuccess) return cuda_fail_c(e, "contract_sum status reset");
     uint32_t* Ap = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + 256);
     uint32_t* Bp = Ap + (uint64_t)F * kTcPlanes * Mp * Kp;
     const uint32_t k_tiles = (uint32_t)(Kp / kTcStageK);
