@@ -1,6 +1,7 @@
 // Device code and the device-facing C ABI of libqtb.so (sm_100a).
 //
-//   K1  qtb_bucket_kernel    one bucket of BucketBackend.process_bucket
+//   K1  qtb_bucket_kernel, qtb_bucket_wide_kernel (large buckets)
+//                            one bucket of BucketBackend.process_bucket
 //                            (qtensor/ProcessingFrameworks.py:29-31,45-147):
 //                            product of the bucket's tensors over the sorted
 //                            union of their variables, summed over variable 0
@@ -1294,105 +1295,150 @@ __device__ __forceinline__ void wide_small(const DevOp* ops, uint32_t lo, uint32
             arena[dst[i]] = (uk[i] & 0x100u) ? make_float2(p0[i].x + p1[i].x, p0[i].y + p1[i].y) : p0[i];
 }
 
-// An operand of a kWideOp item: where its offset moves with the bits that
-// are not in the thread's gathered offset.
+// An operand of a large op: how its offset moves with the bits that are not
+// in the thread's gathered offset.
 struct WideOperand {
     uint32_t sum;    // stride of the summed variable (0: the operand lacks it)
-    uint32_t hi;     // stride of element bit 9
-    uint32_t lo;     // stride of element bit 0 (0 or 1)
-    uint32_t pair;   // bits 0 and the base allow 16-byte loads of element pairs
+    uint32_t hi;     // stride of element bit 9 (0: lacks it)
+    uint32_t kind;   // kWideHi | kWideSum | kWidePair (bit 0, 16-byte loads) or kWideLo (bit 0, 8-byte loads)
+    uint32_t pad;
 };
+constexpr uint32_t kWideHi = 1, kWideSum = 2, kWidePair = 4, kWideLo = 8;
 
-// The four elements of a thread (bits 0 and 9 of the element index) of one
-// operand at p, for the summed variable at 0 (x0) and at 1 (x1).  Every load
-// is issued before any value is used: a stride of 0 loads the same address
-// again (an L1 hit) rather than wait for a value to copy.  The branches are
-// uniform.
-__device__ __forceinline__ void wide_load(const float2* p, const WideOperand& o, float2 (&x0)[4], float2 (&x1)[4]) {
+// The product of a thread's four elements (bits 0 and 9 of the element
+// index), with the summed variable at 0 (p0) and at 1 (p1), times the operand
+// at p.  Only the values that the operand tells apart are loaded, and all of
+// them before any is used: the loads' register bytes, broadcast or not, are
+// what the load/store unit is busy with (74 % of its cycles on a 24-variable
+// bucket while every value was loaded).
+template <bool kFirst, bool kPair, bool kHi, bool kSum, bool kLo>
+__device__ __forceinline__ void wide_product(const float2* p, uint32_t hi, uint32_t sum, float2 (&p0)[4],
+                                             float2 (&p1)[4]) {
     __builtin_assume(__isGlobal(p));
-    const float2* const q[4] = {p, p + o.hi, p + o.sum, p + o.sum + o.hi};
-    if (o.pair) {
-        float4 v[4];
+    constexpr int kH = kHi ? 2 : 1, kS = kSum ? 2 : 1, kE = kPair || kLo ? 2 : 1;
+    float2 v[kS][kH][kE];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(q[i]);
+    for (int s = 0; s < kS; ++s)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            x0[2 * i] = make_float2(v[i].x, v[i].y);
-            x0[2 * i + 1] = make_float2(v[i].z, v[i].w);
-            x1[2 * i] = make_float2(v[2 + i].x, v[2 + i].y);
-            x1[2 * i + 1] = make_float2(v[2 + i].z, v[2 + i].w);
-        }
-    } else {
+        for (int h = 0; h < kH; ++h) {
+            const float2* q = p + (s ? sum : 0u) + (h ? hi : 0u);
+            if constexpr (kPair) {
+                const float4 u = *reinterpret_cast<const float4*>(q);
+                v[s][h][0] = make_float2(u.x, u.y);
+                v[s][h][kE - 1] = make_float2(u.z, u.w);
+            } else {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            x0[2 * i] = *q[i];
-            x1[2 * i] = *q[2 + i];
-        }
-        if (o.lo) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                x0[2 * i + 1] = q[i][1];
-                x1[2 * i + 1] = q[2 + i][1];
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                x0[2 * i + 1] = x0[2 * i];
-                x1[2 * i + 1] = x1[2 * i];
+                for (int e = 0; e < kE; ++e) v[s][h][e] = q[e];
             }
         }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int h = kHi ? e >> 1 : 0, l = kE == 2 ? e & 1 : 0;
+        p0[e] = kFirst ? v[0][h][l] : cmul(p0[e], v[0][h][l]);
+        p1[e] = kFirst ? v[kS - 1][h][l] : cmul(p1[e], v[kS - 1][h][l]);
     }
 }
 
-// What a tile prepares in shared memory for its op.  An operand's offset is
-// a sum over disjoint bits of the element index: the parts of the lane (bits
+template <bool kFirst>
+__device__ __forceinline__ void wide_multiply(const float2* p, const WideOperand& o, float2 (&p0)[4], float2 (&p1)[4]) {
+    // uniform over the CTA
+    switch (o.kind) {
+        case 0: return wide_product<kFirst, false, false, false, false>(p, 0, 0, p0, p1);
+        case kWideHi: return wide_product<kFirst, false, true, false, false>(p, o.hi, 0, p0, p1);
+        case kWideSum: return wide_product<kFirst, false, false, true, false>(p, 0, o.sum, p0, p1);
+        case kWideHi | kWideSum: return wide_product<kFirst, false, true, true, false>(p, o.hi, o.sum, p0, p1);
+        case kWidePair: return wide_product<kFirst, true, false, false, false>(p, 0, 0, p0, p1);
+        case kWidePair | kWideHi: return wide_product<kFirst, true, true, false, false>(p, o.hi, 0, p0, p1);
+        case kWidePair | kWideSum: return wide_product<kFirst, true, false, true, false>(p, 0, o.sum, p0, p1);
+        case kWidePair | kWideHi | kWideSum: return wide_product<kFirst, true, true, true, false>(p, o.hi, o.sum, p0, p1);
+        default: return wide_product<kFirst, false, true, true, true>(p, o.hi, o.sum, p0, p1);
+    }
+}
+
+// What a CTA prepares in shared memory for an op.  An operand's offset is a
+// sum over disjoint bits of the element index: the parts of the lane (bits
 // 1-5) and of the warp (bits 6-8), bits 0 and 9 (WideOperand), and the
 // chunk's part, which the chunk's address holds.
+struct WideOperands {
+    const float2* ptr[kWideMaxK][kWideGroup];
+    uint16_t lane[kWideMaxK][32];
+    uint16_t warp[kWideMaxK][kWideThreads / 32];
+    WideOperand meta[kWideMaxK];
+    uint16_t off[kWideMaxK][kWideThreads];   // the thread's: lane + warp
+};
+
+// An operand as wide_prepare takes it: its descriptor, its first element and
+// whether that is 16-byte aligned.
+struct WideSource {
+    DevIn d;
+    const float2* base;
+    bool aligned;
+};
+
+// Addresses of `chunks` chunks of an op's operands from element j0 on, and
+// with `all` the parts of the offsets that do not change from chunk to chunk
+// (ow: output variables; about one gather per thread for four operands).
+// Every thread calls it; a barrier is passed.
+template <typename Source>
+__device__ __forceinline__ void wide_prepare(WideOperands& s, Source source, uint32_t k, uint32_t ow, bool sum,
+                                             uint32_t j0, uint32_t chunks, bool all) {
+    const uint32_t low = (1u << ow) - 1u, tid = threadIdx.x;
+    const uint32_t fixed = all ? 32u + kWideThreads / 32u + 1u : 0u, each = fixed + chunks;
+    for (uint32_t i = tid; i < k * each; i += kWideThreads) {
+        const uint32_t q = i / each, r = i % each;
+        const WideSource o = source(q);
+        if (r >= fixed) {
+            s.ptr[q][r - fixed] = o.base + gather_bits(j0 + (r - fixed) * kWideChunk, o.d, low);
+        } else if (r < 32u) {
+            s.lane[q][r] = (uint16_t)gather_bits(r << 1, o.d, low);
+        } else if (r < fixed - 1u) {
+            s.warp[q][r - 32u] = (uint16_t)gather_bits((r - 32u) << 6, o.d, low);
+        } else {
+            WideOperand m;
+            m.sum = (sum && ((o.d.mask >> ow) & 1u)) ? 1u << (__popc(o.d.mask) - 1) : 0u;
+            m.hi = ((o.d.mask >> 9) & 1u) << __popc(o.d.mask & 0x1ffu);
+            const bool lo = o.d.mask & 1u;
+            m.kind = lo && !o.aligned ? kWideLo
+                                      : (lo ? kWidePair : 0u) | (m.hi ? kWideHi : 0u) | (m.sum ? kWideSum : 0u);
+            m.pad = 0;
+            s.meta[q] = m;
+        }
+    }
+    __syncthreads();
+    if (all)
+        for (uint32_t q = 0; q < k; ++q) s.off[q][tid] = s.lane[q][tid & 31u] + s.warp[q][tid >> 5];
+}
+
+// Chunk c of a prepared group: the thread's four elements, the products in
+// operand order, summed over the bucket variable when `sum`; `out` is the
+// thread's first element (16-byte aligned when `vec`).
+__device__ __forceinline__ void wide_chunk(const WideOperands& s, uint32_t c, uint32_t k, bool sum, bool vec,
+                                           float2* out) {
+    const uint32_t tid = threadIdx.x;
+    float2 p0[4], p1[4];
+    wide_multiply<true>(s.ptr[0][c] + s.off[0][tid], s.meta[0], p0, p1);
+#pragma unroll 1
+    for (uint32_t q = 1; q < k; ++q) wide_multiply<false>(s.ptr[q][c] + s.off[q][tid], s.meta[q], p0, p1);
+    if (sum)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p0[e] = make_float2(p0[e].x + p1[e].x, p0[e].y + p1[e].y);
+    if (vec) {
+        reinterpret_cast<float4*>(out)[0] = make_float4(p0[0].x, p0[0].y, p0[1].x, p0[1].y);
+        reinterpret_cast<float4*>(out + kWideChunk / 2)[0] = make_float4(p0[2].x, p0[2].y, p0[3].x, p0[3].y);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[(e & 1) + (e >> 1) * (kWideChunk / 2)] = p0[e];
+    }
+}
+
 struct WideShared {
     union {
-        struct {
-            const float2* ptr[kWideMaxK][kWideGroup];
-            uint16_t lane[kWideMaxK][32];
-            uint16_t warp[kWideMaxK][kWideThreads / 32];
-            WideOperand meta[kWideMaxK];
-            uint16_t off[kWideMaxK][kWideThreads];   // the thread's: lane + warp
-        };
+        WideOperands o;                    // a large op's
         uint32_t op_first[kWideSmemOps];   // small ops
     };
     unsigned long long place;   // of the tile to run; 0: no tile left, or the wait ran out
     uint32_t finished, first_place, last;
 };
-
-// Addresses of `chunks` chunks of an op's operands from element j0 on, and
-// with `all` the parts of the offsets that do not change from chunk to chunk;
-// about one gather per thread for four operands.
-__device__ __forceinline__ void wide_prepare(WideShared& s, const DevIn* in, uint32_t k, uint32_t ow, bool sum,
-                                             uint32_t j0, uint32_t chunks, bool all, bool vec, const float2* table,
-                                             const float2* arena) {
-    const uint32_t low = (1u << ow) - 1u;
-    const uint32_t fixed = all ? 32u + kWideThreads / 32u + 1u : 0u, each = fixed + chunks;
-    for (uint32_t i = threadIdx.x; i < k * each; i += kWideThreads) {
-        const uint32_t q = i / each, r = i % each;
-        const DevIn d = ldg_in(in + q);
-        if (r >= fixed) {
-            s.ptr[q][r - fixed] = ((d.src & kSrcTable) ? table + (d.src & ~kSrcTable) : arena + d.src) +
-                                  gather_bits(j0 + (r - fixed) * kWideChunk, d, low);
-        } else if (r < 32u) {
-            s.lane[q][r] = (uint16_t)gather_bits(r << 1, d, low);
-        } else if (r < fixed - 1u) {
-            s.warp[q][r - 32u] = (uint16_t)gather_bits((r - 32u) << 6, d, low);
-        } else {
-            WideOperand o;
-            o.sum = (sum && ((d.mask >> ow) & 1u)) ? 1u << (__popc(d.mask) - 1) : 0u;
-            o.hi = ((d.mask >> 9) & 1u) << __popc(d.mask & 0x1ffu);
-            o.lo = d.mask & 1u;
-            // arena tensors start at multiples of four elements; a gate
-            // table entry may start anywhere
-            o.pair = o.lo && vec && !(d.src & kSrcTable);
-            s.meta[q] = o;
-        }
-    }
-}
 
 // The place of ticket t (one thread; bounded wait until it is filled).
 __device__ unsigned long long wide_place(const WideArgs& w, uint32_t t, int* status) {
@@ -1452,9 +1498,10 @@ __device__ __noinline__ void wide_small_tile(WideShared& s, const uint4* ip, uin
 // while more tiles are ready than CTAs run.  Energies of 3-regular N=256
 // p=4 and Erdos-Renyi N=400 p=3 graphs: 1030 and 1490 us with whole-GPU
 // steps (every tile waited for every network's previous phase, and thread
-// by thread for its own lookups), 432 and 541 us so.  Measured and not
+// by thread for its own lookups), 422 and 505 us so.  Measured and not
 // kept: three CTAs per SM with the next operand's loads in flight (480 and
-// 635 us), the finishing CTA going on with its network's next phase while
+// 635 us), every operand value loaded whether it varies or not (433 and
+// 541 us), the finishing CTA going on with its network's next phase while
 // it holds a ticket (482 and 635 us: the ticket's tile waits for it).
 __global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm) qtb_wide_kernel(const WideArgs w, const RunArgs a) {
     __shared__ WideShared s;
@@ -1486,38 +1533,16 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm) qtb_wide_kernel(
                 const uint32_t k = (i1.y >> 8) & 0xffu;
                 const bool sum = i1.y >> 16;
                 const uint32_t n = min((min(e0 + i2.y, i2.x) - e0) / kWideChunk - c0, kWideGroup);
-                wide_prepare(s, reinterpret_cast<const DevIn*>(plan), k, i1.y & 0xffu, sum, e0 + c0 * kWideChunk, n,
-                             c0 == 0u, w.vec, a.gtable, arena);
-                __syncthreads();
-                if (c0 == 0u)
-                    for (uint32_t q = 0; q < k; ++q) s.off[q][tid] = s.lane[q][tid & 31u] + s.warp[q][tid >> 5];
+                wide_prepare(s.o, [&](uint32_t q) {
+                    const DevIn d = ldg_in(reinterpret_cast<const DevIn*>(plan) + q);
+                    // arena tensors start at multiples of four elements; a
+                    // gate table entry may start anywhere
+                    const bool table = d.src & kSrcTable;
+                    return WideSource{d, table ? a.gtable + (d.src & ~kSrcTable) : arena + d.src, w.vec && !table};
+                }, k, i1.y & 0xffu, sum, e0 + c0 * kWideChunk, n, c0 == 0u);
                 const bool last_group = c0 + kWideGroup >= (min(e0 + i2.y, i2.x) - e0) / kWideChunk;
                 float2* out = arena + i1.x + e0 + c0 * kWideChunk + 2u * tid;
-                for (uint32_t c = 0; c < n; ++c, out += kWideChunk) {
-                    float2 p0[4], p1[4];
-                    wide_load(s.ptr[0][c] + s.off[0][tid], s.meta[0], p0, p1);
-#pragma unroll 1
-                    for (uint32_t q = 1; q < k; ++q) {
-                        float2 x0[4], x1[4];
-                        wide_load(s.ptr[q][c] + s.off[q][tid], s.meta[q], x0, x1);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            p0[e] = cmul(p0[e], x0[e]);
-                            p1[e] = cmul(p1[e], x1[e]);
-                        }
-                    }
-                    if (sum)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) p0[e] = make_float2(p0[e].x + p1[e].x, p0[e].y + p1[e].y);
-                    if (w.vec) {
-                        reinterpret_cast<float4*>(out)[0] = make_float4(p0[0].x, p0[0].y, p0[1].x, p0[1].y);
-                        reinterpret_cast<float4*>(out + kWideChunk / 2)[0] =
-                            make_float4(p0[2].x, p0[2].y, p0[3].x, p0[3].y);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) out[(e & 1) + (e >> 1) * (kWideChunk / 2)] = p0[e];
-                    }
-                }
+                for (uint32_t c = 0; c < n; ++c, out += kWideChunk) wide_chunk(s.o, c, k, sum, w.vec, out);
                 if (last_group) break;
                 __syncthreads();
             }
@@ -1568,6 +1593,47 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm) qtb_wide_kernel(
             reduce_energy_call(a.terms, a.total_jobs, a.energy_groups, a.energy);
             if (tid == 0) *a.done = 0u;   // ready for the next run
         }
+    }
+}
+
+// ----------------------------------------------------------------- K1, large buckets
+// A bucket of at least 2^kBucketWideVars outputs by the chunks of K4: CTAs
+// take contiguous ranges of chunks, the operands' offsets are prepared per
+// group of chunks instead of gathered per element, and pairs of elements
+// load and store 16 bytes.  24 variables (128 MiB): 43.0 -> 32.9 us; a
+// 23-variable bucket of six tensors 61.5 -> 26.4 us.  The line: at 2^16
+// outputs both kernels take 6.2-6.6 us, at 2^17 6.2-8.3 against 4.9-6.2 us,
+// below 2^15 the set-up costs up to 2 us more than it saves.
+constexpr int kBucketWideVars = 17;
+
+__global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm)
+qtb_bucket_wide_kernel(const __grid_constant__ BucketArgs a, const uint32_t chunks_per_cta) {
+    __shared__ WideOperands s;
+    const uint32_t chunks = (1u << a.w) / kWideChunk;
+    const uint32_t first = blockIdx.x * chunks_per_cta, end = min(first + chunks_per_cta, chunks);
+    const bool vec = reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
+    for (uint32_t c0 = first; c0 < end; c0 += kWideGroup) {
+        const uint32_t n = min(end - c0, kWideGroup);
+        if (c0 != first) __syncthreads();
+        wide_prepare(s, [&](uint32_t q) {
+            DevIn d;
+            d.mask = a.mask[q];
+            d.src = 0;
+            d.runs = a.runs[q];
+            return WideSource{d, a.in[q], reinterpret_cast<uintptr_t>(a.in[q]) % 16 == 0};
+        }, (uint32_t)a.k, (uint32_t)a.w, a.sum != 0, c0 * kWideChunk, n, c0 == first);
+        float2* out = a.out + (size_t)c0 * kWideChunk + 2u * threadIdx.x;
+        for (uint32_t c = 0; c < n; ++c, out += kWideChunk) wide_chunk(s, c, (uint32_t)a.k, a.sum != 0, vec, out);
+    }
+}
+
+static void launch_bucket(const BucketArgs& a, cudaStream_t st) {
+    if (a.w >= kBucketWideVars && a.w < 32) {
+        const uint32_t chunks = (1u << a.w) / kWideChunk;
+        const uint32_t per = (chunks + 148 * kWideCtasPerSm - 1) / (148 * kWideCtasPerSm);
+        qtb_bucket_wide_kernel<<<(chunks + per - 1) / per, kWideThreads, 0, st>>>(a, per);
+    } else {
+        qtb_bucket_kernel<<<bucket_blocks(a.w), kBucketThreads, 0, st>>>(a);
     }
 }
 
@@ -2535,7 +2601,7 @@ int qtb_bucket_c64(const qtb_bucket_desc* d, const void* const* inputs, void* ou
     a.k = d->n_inputs;
     a.sum = d->sum_first;
     a.w = d->n_vars - d->sum_first;
-    qtb_bucket_kernel<<<bucket_blocks(a.w), kBucketThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    launch_bucket(a, static_cast<cudaStream_t>(stream));
     QTB_CUDA(cudaGetLastError());
     return QTB_OK;
 }
@@ -3116,7 +3182,7 @@ int qtb_plan_run_plain(qtb_plan* plan, int32_t first, int32_t count, const doubl
             a.k = op.k;
             a.sum = op.sum;
             a.w = op.u - op.sum;
-            qtb_bucket_kernel<<<bucket_blocks(a.w), kBucketThreads, 0, st>>>(a);
+            launch_bucket(a, st);
             QTB_CUDA(cudaGetLastError());
         }
         const float2* res = (net.result_src & kSrcTable) ? table + (net.result_src & ~kSrcTable)
