@@ -93,7 +93,8 @@ int qtb_bucket_c64(const qtb_bucket_desc* desc, const void* const* inputs,
  * K >= 32 and M, N >= 64): complex products in 3xTF32 (each operand split
  * into TF32 high and low parts), FP32 accumulation in tensor memory per
  * 32-k block, the blocks summed in FP32 registers with round-to-nearest,
- * 128 x 64 complex output tiles; else (mode 1, or mode 0 for smaller shapes) on the CUDA
+ * 128 x 64 or 128 x 128 complex output tiles, a long K in up to eight parts
+ * summed in order; else (mode 1, or mode 0 for smaller shapes) on the CUDA
  * cores in FP32.  scratch (qtb_contract_sum_scratch_bytes for the same
  * shape and mode) holds the split operands; its first 4 bytes are a status
  * word, 0 after a good run, 2 when a staging copy or the MMAs did not
@@ -320,9 +321,9 @@ int qtb_plan_run_plain(qtb_plan* plan, int32_t first, int32_t count, const doubl
  * QTB_SCHEDULE fixes the schedule.                                       */
 int qtb_plan_set_autotune(qtb_plan* plan, int32_t enable);
 /* Halves of every SM that the plan's wide waves may hold (0, the default:
- * both; a half is two CTAs of 256 threads).  A wave keeps its CTAs for its whole run; with 1, half of
- * every SM stays free for other streams' kernels (a server's concurrent
- * requests) while a wide request runs.  Set before a range's first run.  */
+ * both; a half is two CTAs of 256 threads).  A wave keeps its CTAs for its
+ * whole run; with 1, half of every SM stays free for other streams' kernels
+ * (a server's concurrent requests) while a wide request runs.  Set before a range's first run.  */
 int qtb_plan_set_wave_ctas_per_sm(qtb_plan* plan, int32_t ctas);
 /* How the CTAs of a persistent launch take networks.  0 (the default): a
  * CTA's first network is the job of its own index, later ones come from

@@ -10,27 +10,26 @@
 // a large summed dimension it runs on the tcgen05 tensor cores:
 //   * a pre-pass splits every operand into TF32 "hi" (rounded to nearest,
 //     cvt.rna.tf32.f32) and "lo" (the rounded remainder) planes of the real
-//     and imaginary parts, transposed to K-major and tiled 128 (or 64) rows
-//     x 16 k in the canonical no-swizzle core-matrix layout (8 rows x 16
-//     bytes), zero padded to whole 32-k blocks;
-//   * one CTA per (f, 128 x 64 output tile): one lane stages the eight
-//     planes of each 16-k tile (8 KB of A, 4 KB of B each) into one of two
-//     shared-memory stages with bulk copies (cp.async.bulk, mbarrier
-//     transaction count, bounded wait), and issues tcgen05.mma kind::tf32
-//     (M=128, N=64, K=8) into Re and Im accumulators in TMEM, FP32, while
-//     the next tile's copy lands:
-//       Re += Ar_hi Br_hi + Ar_hi Br_lo + Ar_lo Br_hi - (Ai_hi Bi_hi + Ai_hi Bi_lo + Ai_lo Bi_hi)
-//       Im += Ar_hi Bi_hi + Ar_hi Bi_lo + Ar_lo Bi_hi + Ai_hi Br_hi + Ai_hi Br_lo + Ai_lo Br_hi
-//     (3xTF32: Ootomo and Yokota, "Recovering single precision accuracy from
-//     Tensor Cores while surpassing the FP32 theoretical peak performance",
-//     IJHPCA 2022; the lo x lo term is dropped), the negative terms through
-//     the instruction descriptor's negate-A bit;
-//   * every 32-k block goes to one of two TMEM buffers from zero; four warps
-//     read a finished buffer back (tcgen05.ld) and add it into FP32
+//     and imaginary parts, transposed to K-major and tiled 128 rows (of A) or
+//     kN columns (of B) x 8 k in the canonical no-swizzle core-matrix layout
+//     (8 rows x 16 bytes), zero padded to whole 32-k blocks;
+//   * a cluster of 1 to 8 CTAs per (f, 128 x kN output tile), kN 64 or 128,
+//     each CTA a contiguous part of the 32-k blocks: one lane stages tiles
+//     with bulk copies (cp.async.bulk, mbarrier transaction count, bounded
+//     waits), another issues tcgen05.mma kind::tf32 (M=128, N=2 kN, K=8) into
+//     [Re | Im] accumulators in TMEM, FP32, while later tiles' copies land:
+//       [Re | Im] += (Ar_hi + Ar_lo)[Br | Bi] + (Ai_hi + Ai_lo)[-Bi | Br]
+//     with B split alike and the lo x lo terms dropped (3xTF32: Ootomo and
+//     Yokota, "Recovering single precision accuracy from Tensor Cores while
+//     surpassing the FP32 theoretical peak performance", IJHPCA 2022); B's
+//     rows are stored once as [-Bi | Br | Bi], which holds both operands;
+//   * every 32-k block goes to one of two TMEM buffers from zero; epilogue
+//     warps read a finished buffer back (tcgen05.ld) and add it into FP32
 //     registers with round-to-nearest while the next block fills the other
 //     buffer, since the tensor cores' own accumulation rounds toward zero
 //     (Ootomo and Yokota keep the long sum outside the tensor cores for the
-//     same reason); the registers are written as complex64.
+//     same reason); the CTAs' sums meet in shared memory, in rank order, and
+//     leave as whole rows of complex64.
 // With a small summed dimension (the reference's own buckets sum one binary
 // index, K = 2) a tile would be mostly padding, and a CUDA-core kernel
 // computes the same sums in FP32.
@@ -222,30 +221,36 @@ static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 1
 
 // ----------------------------------------------------------------- tensor cores
 constexpr uint32_t kTcM = 128;                        // output tile rows (A tile rows)
-constexpr uint32_t kTcN = 64;                         // output tile columns (complex)
-constexpr uint32_t kTcBRows = 2 * kTcN;               // B tile rows: [Br | Bi] or [-Bi | Br]
 constexpr uint32_t kTcK = 32;                         // k per accumulation block (K padded to it)
 constexpr uint32_t kTcStageK = 8;                     // k per staged tile (one MMA k step)
-constexpr uint32_t kTcStages = 3;                     // shared-memory stages (two copies in flight)
 constexpr uint32_t kTcStagesPerBlock = kTcK / kTcStageK;
+constexpr uint32_t kTcAPlanes = 4;                    // Ar_hi Ar_lo Ai_hi Ai_lo
+constexpr uint32_t kTcBPlanes = 2;                    // [-Bi | Br | Bi]: hi, lo
 constexpr uint32_t kTcAWords = kTcM * kTcStageK;      // 1024 x 32-bit = 4 KB per A plane and stage
-constexpr uint32_t kTcBWords = kTcBRows * kTcStageK;  // 1024 x 32-bit = 4 KB per B plane and stage
-constexpr uint32_t kTcPlanes = 4;                     // A: re_hi re_lo im_hi im_lo; B: B1_hi B1_lo B2_hi B2_lo
-constexpr uint32_t kTcStageWords = kTcPlanes * (kTcAWords + kTcBWords);   // 32 KB per stage
 constexpr uint32_t kTcChunks = kTcStageK / 4;         // 16-byte k chunks per row of a tile
-constexpr uint32_t kTcEpilogueWarps = 4;              // one per 32 TMEM lanes of the 128-row tile
-constexpr uint32_t kTcThreads = 32 * (kTcEpilogueWarps + 1);   // + the copy/MMA issuing warp
-constexpr uint32_t kTcBufCols = 2 * kTcN;             // one accumulator buffer: Re 0..63, Im 64..127
-constexpr uint32_t kTcTmemCols = 2 * kTcBufCols;      // two buffers
 constexpr uint32_t kTcSpinLimit = 1u << 24;           // bounded mbarrier waits (~1 s)
 constexpr int kTcStatusTimeout = 2;
 
-// Word of element (r, k) inside a tile of kTcStageK k: core matrix (row
-// group r / 8, k chunk k / 4) at (g * kTcChunks + c) * 32 words, 8 rows of
-// 16 bytes each.
-__device__ __forceinline__ uint32_t tc_tile_word(uint32_t r, uint32_t k) {
-    return (((r >> 3) * kTcChunks + (k >> 2)) << 5) + ((r & 7u) << 2) + (k & 3u);
-}
+// What depends on the output tile's columns kN (complex).
+template <uint32_t kN>
+struct TcTile {
+    static constexpr uint32_t kBWords = 3 * kN * kTcStageK;                        // per B plane and stage
+    static constexpr uint32_t kStageWords = kTcAPlanes * kTcAWords + kTcBPlanes * kBWords;   // 40 or 28 KB
+    static constexpr uint32_t kStages = kN == 128 ? 5 : 7;                         // about 200 KB
+    static constexpr uint32_t kEpilogueWarps = kN / 16;                            // 64 columns x 32 rows each
+    static constexpr uint32_t kThreads = 32 * (kEpilogueWarps + 2);                // + the MMA and the copy warp
+    static constexpr uint32_t kBufCols = 2 * kN;                                   // one accumulator buffer [Re | Im]
+    static constexpr uint32_t kTmemCols = 2 * kBufCols;
+    // instruction descriptor: FP32 accumulator, TF32 A and B, both K-major,
+    // N = 2 kN (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
+    static constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((2 * kN >> 3) << 17) | ((kTcM >> 4) << 24);
+    // the finished tile in the stages' place: rows of kN complex64, padded by
+    // 16 bytes so that the rows of a warp's lanes start on different banks
+    static constexpr uint32_t kRowBytes = kN * 8 + 16;
+    static constexpr size_t kBarOffset = (size_t)kStages * kStageWords * 4;
+    static constexpr size_t kSmemBytes = kBarOffset + (2 * kStages + 4) * 8 + 16;
+    static_assert(kTcM * kRowBytes <= kBarOffset, "the tile fits the stages");
+};
 
 __device__ __forceinline__ uint32_t tf32_round(float x) {
     uint32_t r;
@@ -259,74 +264,73 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) 
     lo = tf32_round(x - __uint_as_float(hi));
 }
 
-// Copies a staged tile (`words` 32-bit words) from shared memory to dst, 16 bytes per thread and step.
-__device__ __forceinline__ void tc_write_tile(const uint32_t* s, uint32_t* dst, uint32_t words) {
-    const uint4* in = reinterpret_cast<const uint4*>(s);
-    uint4* out = reinterpret_cast<uint4*>(dst);
-    for (uint32_t i = threadIdx.x; i < words / 4; i += blockDim.x) out[i] = in[i];
+// TF32 hi / lo of four k of one row: one 16-byte chunk of a core matrix each.
+__device__ __forceinline__ void tf32_split4(const float (&x)[4], uint4& hi, uint4& lo) {
+    tf32_split(x[0], hi.x, lo.x);
+    tf32_split(x[1], hi.y, lo.y);
+    tf32_split(x[2], hi.z, lo.z);
+    tf32_split(x[3], hi.w, lo.w);
 }
 
-// A[k][f][m] (complex64, M rows) -> TF32 planes Ar_hi, Ar_lo, Ai_hi, Ai_lo
-// in tiles of 128 rows x kTcStageK k, ordered (f, row tile, k tile), each
-// tile's four planes consecutive, so that one bulk copy stages all four.
-// One block per tile: coalesced reads of the tile's rows, the split into
-// shared memory in the core-matrix layout, then one contiguous write.
-__global__ void __launch_bounds__(256) qtb_tc_split_kernel(const float2* __restrict__ src,
-                                                           uint32_t* __restrict__ dst, uint32_t K, uint32_t F,
-                                                           uint32_t M, uint32_t Mp, uint32_t Kp) {
-    __shared__ __align__(16) uint32_t s[kTcPlanes * kTcAWords];
-    const uint32_t k_tiles = Kp / kTcStageK, row_tiles = Mp / kTcM;
-    const uint32_t bid = blockIdx.x;
-    const uint32_t kt = bid % k_tiles, rt = (bid / k_tiles) % row_tiles, f = bid / (k_tiles * row_tiles);
-    for (uint32_t e = threadIdx.x; e < kTcM * kTcStageK; e += blockDim.x) {
-        const uint32_t r = e % kTcM, k = e / kTcM;
-        const uint32_t m = rt * kTcM + r, kk = kt * kTcStageK + k;
-        const float2 v = (m < M && kk < K) ? src[((uint64_t)kk * F + f) * M + m] : make_float2(0.f, 0.f);
-        uint32_t rh, rl, ih, il;
-        tf32_split(v.x, rh, rl);
-        tf32_split(v.y, ih, il);
-        const uint32_t w = tc_tile_word(r, k);
-        s[w] = rh;
-        s[kTcAWords + w] = rl;
-        s[2 * kTcAWords + w] = ih;
-        s[3 * kTcAWords + w] = il;
+// The planes of A and of B.  A[k][f][m] -> tiles of 128 rows x 8 k, ordered
+// (f, row tile, k tile), the four planes of a tile consecutive, so that one
+// bulk copy stages all four; B[k][f][n] -> tiles of kN columns x 8 k, ordered
+// (f, column tile, k tile), two planes of rows [-Bi | Br | Bi] (the negation
+// is exact in TF32).  A thread takes four k of one row or column: its reads
+// are coalesced over the rows, and its 16-byte writes fill 128-byte lines of
+// eight rows, so nothing is exchanged between threads.  Element (r, k) of a
+// plane: core matrix (r / 8, k / 4), 8 rows of 16 bytes each.  The first
+// blocks split A, the others B; the status word is cleared for the kernel
+// that follows.
+template <uint32_t kN>
+__global__ void __launch_bounds__(256) qtb_tc_split_kernel(const float2* __restrict__ A, const float2* __restrict__ B,
+                                                           uint4* __restrict__ Ap, uint4* __restrict__ Bp, uint32_t K,
+                                                           uint32_t F, uint32_t M, uint32_t N, uint32_t k_tiles,
+                                                           uint32_t row_tiles, uint32_t col_tiles, uint32_t a_blocks,
+                                                           int* status) {
+    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
+    const bool is_a = blockIdx.x < a_blocks;
+    const uint32_t rows = is_a ? kTcM : kN, tiles = is_a ? row_tiles : col_tiles, width = is_a ? M : N;
+    const uint64_t unit = (uint64_t)(is_a ? blockIdx.x : blockIdx.x - a_blocks) * 256u + threadIdx.x;
+    const uint32_t r = (uint32_t)(unit % rows), c = (uint32_t)(unit / rows) % kTcChunks;
+    const uint64_t tile = unit / (rows * kTcChunks);
+    if (tile >= (uint64_t)F * tiles * k_tiles) return;
+    const uint32_t kt = (uint32_t)(tile % k_tiles), rt = (uint32_t)(tile / k_tiles % tiles);
+    const uint64_t f = tile / k_tiles / tiles;
+    const uint64_t col = (uint64_t)rt * rows + r;
+    const float2* src = is_a ? A : B;
+    float re[4], im[4];
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+        const uint64_t kk = (uint64_t)kt * kTcStageK + 4u * c + e;
+        const float2 v = (col < width && kk < K) ? src[(kk * F + f) * width + col] : make_float2(0.f, 0.f);
+        re[e] = v.x;
+        im[e] = v.y;
     }
-    __syncthreads();
-    tc_write_tile(s, dst + (uint64_t)bid * kTcPlanes * kTcAWords, kTcPlanes * kTcAWords);
-}
-
-// B[k][f][n] (complex64, N columns) -> TF32 planes B1_hi, B1_lo, B2_hi,
-// B2_lo in tiles of 128 rows x kTcStageK k, ordered (f, output column
-// tile, k tile), each tile's four planes consecutive: in the rows of tile
-// t, B1 holds Br of columns 64 t .. 64 t + 63 then their Bi, and B2 holds
-// -Bi then Br (the negation is exact in TF32).  One block per tile, as for A.
-__global__ void __launch_bounds__(256) qtb_tc_split_b_kernel(const float2* __restrict__ src,
-                                                             uint32_t* __restrict__ dst, uint32_t K, uint32_t F,
-                                                             uint32_t N, uint32_t Np, uint32_t Kp) {
-    __shared__ __align__(16) uint32_t s[kTcPlanes * kTcBWords];
-    const uint32_t k_tiles = Kp / kTcStageK, col_tiles = Np / kTcN;
-    const uint32_t bid = blockIdx.x;
-    const uint32_t kt = bid % k_tiles, t = (bid / k_tiles) % col_tiles, f = bid / (k_tiles * col_tiles);
-    for (uint32_t e = threadIdx.x; e < kTcN * kTcStageK; e += blockDim.x) {
-        const uint32_t j = e % kTcN, k = e / kTcN;
-        const uint32_t n = t * kTcN + j, kk = kt * kTcStageK + k;
-        const float2 v = (n < N && kk < K) ? src[((uint64_t)kk * F + f) * N + n] : make_float2(0.f, 0.f);
-        uint32_t rh, rl, ih, il;
-        tf32_split(v.x, rh, rl);
-        tf32_split(v.y, ih, il);
-        const uint32_t w_re = tc_tile_word(j, k);          // row j: Br (B1), -Bi (B2)
-        const uint32_t w_im = tc_tile_word(j + kTcN, k);   // row 64 + j: Bi (B1), Br (B2)
-        s[w_re] = rh;
-        s[kTcBWords + w_re] = rl;
-        s[w_im] = ih;
-        s[kTcBWords + w_im] = il;
-        s[2 * kTcBWords + w_re] = ih ^ 0x80000000u;
-        s[3 * kTcBWords + w_re] = il ^ 0x80000000u;
-        s[2 * kTcBWords + w_im] = rh;
-        s[3 * kTcBWords + w_im] = rl;
+    uint4 rh, rl, ih, il;
+    tf32_split4(re, rh, rl);
+    tf32_split4(im, ih, il);
+    auto chunk = [&](uint32_t row) { return ((row >> 3) * kTcChunks + c) * 8u + (row & 7u); };
+    if (is_a) {
+        constexpr uint32_t kPlane = kTcAWords / 4;
+        uint4* dst = Ap + tile * (kTcAPlanes * kPlane) + chunk(r);
+        dst[0] = rh;
+        dst[kPlane] = rl;
+        dst[2 * kPlane] = ih;
+        dst[3 * kPlane] = il;
+    } else {
+        constexpr uint32_t kPlane = TcTile<kN>::kBWords / 4;
+        auto negated = [](uint4 v) {
+            return make_uint4(v.x ^ 0x80000000u, v.y ^ 0x80000000u, v.z ^ 0x80000000u, v.w ^ 0x80000000u);
+        };
+        uint4* dst = Bp + tile * (kTcBPlanes * kPlane);
+        dst[chunk(r)] = negated(ih);
+        dst[chunk(kN + r)] = rh;
+        dst[chunk(2 * kN + r)] = ih;
+        dst[kPlane + chunk(r)] = negated(il);
+        dst[kPlane + chunk(kN + r)] = rl;
+        dst[kPlane + chunk(2 * kN + r)] = il;
     }
-    __syncthreads();
-    tc_write_tile(s, dst + (uint64_t)bid * kTcPlanes * kTcBWords, kTcPlanes * kTcBWords);
 }
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) {
@@ -340,10 +344,6 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) |
            ((uint64_t)(kTcChunks * 128u >> 4) << 32) | (uint64_t(1) << 46);
 }
-
-// Instruction descriptor: FP32 accumulator, TF32 A and B, both K-major,
-// N = 64 (>> 3 at bit 17), M = 128 (>> 4 at bit 24); bit 13 negates A.
-constexpr uint32_t kTcIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kTcBRows >> 3) << 17) | ((kTcM >> 4) << 24);
 
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
@@ -366,24 +366,31 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
-// Eight 32-bit TMEM columns of this thread's lane at each of two
-// addresses, one wait for both loads; the wait is in the same asm as the
-// loads, so no use of the registers can be scheduled before it.
-__device__ __forceinline__ void tc_ld2x8(uint32_t ta, uint32_t tb, float* a, float* b) {
-    uint32_t r[16];
+// 32 32-bit TMEM columns of this thread's lane at each of two addresses,
+// one wait for both loads (a load's latency, not its width, is what costs
+// while the MMAs run); the wait is in the same asm as the loads, so no use of
+// the registers can be scheduled before it.
+__device__ __forceinline__ void tc_ld2x32(uint32_t ta, uint32_t tb, uint32_t (&r)[64]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,"
+        "%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,"
+        "%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,"
+        "%40,%41,%42,%43,%44,%45,%46,%47,"
+        "%48,%49,%50,%51,%52,%53,%54,%55,"
+        "%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+          "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+          "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+          "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+          "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
         : "r"(ta), "r"(tb)
         : "memory");
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        a[j] = __uint_as_float(r[j]);
-        b[j] = __uint_as_float(r[8 + j]);
-    }
 }
 
 __device__ __forceinline__ void tc_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -397,35 +404,50 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
                  : "memory");
 }
 
-// One CTA per (f, 128 x 64 tile of C), five warps.  Ap / Bp: the pre-pass
-// planes, in tiles of kTcStageK k.
-//   * Warp 4 (one elected lane) stages tiles with bulk copies into
-//     kTcStages shared-memory stages, kTcStages - 1 tiles ahead of the
-//     MMAs it issues, so that copies land while earlier tiles' MMAs run.
-//     kTcStagesPerBlock tiles make one 32-k block, accumulated in one of two
-//     TMEM buffers from zero.
-//   * Warps 0-3 (one per 32 TMEM lanes) read a finished block's buffer
-//     with tcgen05.ld and add it into FP32 registers with round-to-nearest
-//     (the tensor cores' own accumulation rounds toward zero, which over a
-//     long k range biases the sum: about 3e-5 relative at K = 1000), while
-//     the next block's MMAs fill the other buffer.
+// Cluster of `split` CTAs (grid x = column tiles x split) per (f, 128 x kN
+// tile of C); CTA `rank` takes its part of the 32-k blocks.
+//   * One lane of the last warp stages tiles with bulk copies into kStages
+//     shared-memory stages as they come free; one lane of the warp before it
+//     issues the MMAs and never waits for one (a single lane doing both
+//     waited for each tile's MMAs to refill its stage: 1150 of the 1550
+//     cycles per tile, whatever the tile's MMAs).  kTcStagesPerBlock tiles
+//     make one 32-k block, accumulated in one of two TMEM buffers from zero.
+//   * The epilogue warps (32 TMEM lanes x 64 columns each) read a finished
+//     block's buffer with tcgen05.ld and add it into FP32 registers with
+//     round-to-nearest (the tensor cores' own accumulation rounds toward
+//     zero, which over a long k range biases the sum: about 3e-5 relative at
+//     K = 1000), while the next block's MMAs fill the other buffer.
 // mbarriers: full[s] (stage s landed), empty[s] (stage s's MMAs done),
-// tfull[b] (buffer b's block done), tempty[b] (buffer b read, 128
-// arrivals).  Every wait is bounded; on a timeout the status word is set,
-// every role stops, and the CTA waits (bounded, in phase order) for its
-// copies and MMAs in flight before freeing TMEM.
-__global__ void __launch_bounds__(kTcThreads, 2)
+// tfull[b] (buffer b's block done), tempty[b] (buffer b read by every
+// epilogue thread).  Every wait is bounded; on a timeout the status word is
+// set, every role stops, and the CTA waits (bounded, in phase order) for its
+// copies and MMAs in flight before freeing TMEM; it still meets its
+// cluster's barriers.
+// What bounds it: shared memory.  A 128 x 128 tile's six MMAs take 768 tensor
+// cycles per 8 k, read 72 KB of operands and see 40 KB written: 875 cycles at
+// 128 bytes each (measured about 1100).  128 x 64 tiles with B stored as both
+// [Br | Bi] and [-Bi | Br] also pulled 32 KB per 384 cycles through L2.
+// K=1024, F=2, M=N=1024: 165 -> 106 us; K=500, F=3, M=333, N=190: 71 -> 23 us
+// (4 CTAs per tile in place of 27 serial ones).  Measured and not kept: B as
+// [Br | Bi] with the negative products through the descriptor's negate-A bit
+// (32 KB per tile but N = 128 MMAs, 128 operand bytes per cycle: 116 us).
+template <uint32_t kN>
+__global__ void __launch_bounds__(TcTile<kN>::kThreads, 1)
 qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restrict__ Bp, float2* __restrict__ C,
-                       uint32_t F, uint32_t M, uint32_t N, uint32_t Mp, uint32_t Np, uint32_t Kp, int* status) {
-    constexpr uint32_t NS = kTcStages;
+                       uint32_t M, uint32_t N, uint32_t row_tiles, uint32_t col_tiles, uint32_t k_blocks,
+                       uint32_t split, uint32_t vec, int* status) {
+    using T = TcTile<kN>;
+    constexpr uint32_t NS = T::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];
-    // [stage 0: A planes x4 | B planes x4][stage 1] ..., the mbarriers, the TMEM slot
+    // [stage 0: A planes x4 | B planes x2][stage 1] ..., the mbarriers, the TMEM slot
     uint32_t* stages = reinterpret_cast<uint32_t*>(smem);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(stages + NS * kTcStageWords);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::kBarOffset);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NS + 4);
     __shared__ volatile int s_ok;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t nt = blockIdx.x, mt = blockIdx.y, f = blockIdx.z;
+    const uint32_t nt = blockIdx.x / split, rank = blockIdx.x % split, mt = blockIdx.y, f = blockIdx.z;
+    const uint32_t block0 = k_blocks * rank / split, n_blocks = k_blocks * (rank + 1) / split - block0;
+    const uint32_t n_tiles = n_blocks * kTcStagesPerBlock;
     auto full = [&](uint32_t s) { return tc_smem(&bars[s]); };
     auto empty = [&](uint32_t s) { return tc_smem(&bars[NS + s]); };
     auto tfull = [&](uint32_t b) { return tc_smem(&bars[2 * NS + b]); };
@@ -434,43 +456,57 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
         for (uint32_t i = 0; i < 2 * NS + 2; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[i])));
         for (uint32_t b = 0; b < 2; ++b)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tempty(b)), "r"(32 * kTcEpilogueWarps));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tempty(b)), "r"(32 * T::kEpilogueWarps));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_ok = 1;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_slot)),
-                     "r"(kTcTmemCols));
+                     "r"(T::kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
-    const uint32_t n_tiles = Kp / kTcStageK, n_blocks = Kp / kTcK;
+    // launched while the split kernel still runs: its planes and the status
+    // word are ready from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     auto fail_once = [&]() {
         if (s_ok) atomicOr(status, kTcStatusTimeout);
         s_ok = 0;
     };
-    if (warp == kTcEpilogueWarps) {
+    float acc_re[64], acc_im[64];
+    if (warp == T::kEpilogueWarps + 1) {   // the copies
         if (lane == 0) {
             // this CTA's tiles: (f, row tile, k tile) of A, (f, column tile, k tile) of B
-            const uint32_t* a_f = Ap + ((uint64_t)f * (Mp / kTcM) + mt) * n_tiles * (kTcPlanes * kTcAWords);
-            const uint32_t* b_f = Bp + ((uint64_t)f * (Np / kTcN) + nt) * n_tiles * (kTcPlanes * kTcBWords);
-            auto stage_a = [&](uint32_t s) { return tc_smem(stages + s * kTcStageWords); };
-            auto stage_b = [&](uint32_t s) { return tc_smem(stages + s * kTcStageWords + kTcPlanes * kTcAWords); };
-            auto load = [&](uint32_t i) {   // tile i into stage i % NS
-                const uint32_t s = i % NS;
+            const uint64_t k_tiles = (uint64_t)k_blocks * kTcStagesPerBlock, kt0 = (uint64_t)block0 * kTcStagesPerBlock;
+            const uint32_t* a_f = Ap + (((uint64_t)f * row_tiles + mt) * k_tiles + kt0) * (kTcAPlanes * kTcAWords);
+            const uint32_t* b_f = Bp + (((uint64_t)f * col_tiles + nt) * k_tiles + kt0) * (kTcBPlanes * T::kBWords);
+            uint32_t loaded = 0;
+            for (; loaded < n_tiles && s_ok; ++loaded) {   // tile `loaded` into stage loaded % NS
+                const uint32_t s = loaded % NS;
+                if (loaded >= NS && !tc_wait(empty(s), (loaded / NS - 1u) & 1u)) {
+                    fail_once();   // the MMAs have not read the stage's previous tile
+                    break;
+                }
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full(s)),
-                             "r"(kTcStageWords * 4u)
+                             "r"(T::kStageWords * 4u)
                              : "memory");
-                // the tile's four planes are consecutive in global memory and in the stage
-                tc_bulk(stage_a(s), a_f + (uint64_t)i * kTcPlanes * kTcAWords, kTcPlanes * kTcAWords * 4u, full(s));
-                tc_bulk(stage_b(s), b_f + (uint64_t)i * kTcPlanes * kTcBWords, kTcPlanes * kTcBWords * 4u, full(s));
-            };
-            uint32_t loaded = 0, landed = 0;   // tiles whose copies were issued, waited for
-            uint32_t committed[NS] = {}, retired[NS] = {};   // empty[s] phases issued, waited for
-            for (; loaded < NS - 1 && loaded < n_tiles; ++loaded) load(loaded);
+                // the tile's planes are consecutive in global memory and in the stage
+                const uint32_t dst = tc_smem(stages + s * T::kStageWords);
+                tc_bulk(dst, a_f + (uint64_t)loaded * kTcAPlanes * kTcAWords, kTcAPlanes * kTcAWords * 4u, full(s));
+                tc_bulk(dst + kTcAPlanes * kTcAWords * 4u, b_f + (uint64_t)loaded * kTcBPlanes * T::kBWords,
+                        kTcBPlanes * T::kBWords * 4u, full(s));
+            }
+            // no copy may still write shared memory when it is reused: wait
+            // (bounded) for each stage's last one
+            for (uint32_t i = loaded > NS ? loaded - NS : 0u; i < loaded; ++i) tc_wait(full(i % NS), (i / NS) & 1u);
+        }
+        __syncwarp();
+    } else if (warp == T::kEpilogueWarps) {   // the MMAs
+        if (lane == 0) {
+            uint32_t committed = 0;
             for (uint32_t i = 0; i < n_tiles && s_ok; ++i) {
                 const uint32_t s = i % NS, b = i / kTcStagesPerBlock, buf = b & 1u;
                 const bool block_first = i % kTcStagesPerBlock == 0;
@@ -482,55 +518,36 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
                     fail_once();
                     break;
                 }
-                landed = i + 1;
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                // planes: A 0 Ar_hi 1 Ar_lo 2 Ai_hi 3 Ai_lo | B 0 B1_hi 1 B1_lo 2 B2_hi 3 B2_lo with
-                // B1 = [Br | Bi] and B2 = [-Bi | Br] along N, so that
-                // Ar B1 + Ai B2 = [Re | Im] in the buffer's 128 columns
-                const uint32_t abase = stage_a(s), bbase = stage_b(s);
-                const uint32_t acc = tmem + buf * kTcBufCols;
-#pragma unroll
-                for (uint32_t ks = 0; ks < kTcStageK / 8; ++ks) {
-                    auto da = [&](uint32_t q) { return tc_desc(abase + q * kTcAWords * 4u + ks * 256u); };
-                    auto db = [&](uint32_t q) { return tc_desc(bbase + q * kTcBWords * 4u + ks * 256u); };
-                    const uint32_t first = (block_first && ks == 0) ? 0u : 1u;   // a block starts from zero
-                    tc_mma(acc, da(0), db(0), kTcIdesc, first);
-                    tc_mma(acc, da(0), db(1), kTcIdesc, 1u);
-                    tc_mma(acc, da(1), db(0), kTcIdesc, 1u);
-                    tc_mma(acc, da(2), db(2), kTcIdesc, 1u);
-                    tc_mma(acc, da(2), db(3), kTcIdesc, 1u);
-                    tc_mma(acc, da(3), db(2), kTcIdesc, 1u);
-                }
+                // A planes: 0 Ar_hi 1 Ar_lo 2 Ai_hi 3 Ai_lo.  B rows [-Bi | Br | Bi]:
+                // from row kN on [Br | Bi], from row 0 on [-Bi | Br]
+                const uint32_t abase = tc_smem(stages + s * T::kStageWords), bbase = abase + kTcAPlanes * kTcAWords * 4u;
+                const uint32_t acc = tmem + buf * T::kBufCols;
+                auto da = [&](uint32_t q) { return tc_desc(abase + q * kTcAWords * 4u); };
+                auto db = [&](uint32_t q, uint32_t row) {
+                    return tc_desc(bbase + q * T::kBWords * 4u + row * (kTcStageK * 4u));
+                };
+                tc_mma(acc, da(0), db(0, kN), T::kIdesc, block_first ? 0u : 1u);   // a block starts from zero
+                tc_mma(acc, da(0), db(1, kN), T::kIdesc, 1u);
+                tc_mma(acc, da(1), db(0, kN), T::kIdesc, 1u);
+                tc_mma(acc, da(2), db(0, 0), T::kIdesc, 1u);
+                tc_mma(acc, da(2), db(1, 0), T::kIdesc, 1u);
+                tc_mma(acc, da(3), db(0, 0), T::kIdesc, 1u);
                 tc_commit(empty(s));
-                ++committed[s];
+                committed = i + 1;
                 if (i % kTcStagesPerBlock == kTcStagesPerBlock - 1) tc_commit(tfull(buf));
-                // tile i + NS - 1 goes into the stage of tile i - 1 once that
-                // tile's MMAs are done; it lands while later tiles' MMAs run
-                if (loaded < n_tiles) {
-                    if (i >= 1) {
-                        const uint32_t sp = (i - 1) % NS;
-                        if (!tc_wait(empty(sp), ((i - 1) / NS) & 1u)) {
-                            fail_once();
-                            break;
-                        }
-                        ++retired[sp];
-                    }
-                    load(loaded++);
-                }
             }
-            // nothing of this CTA may still write shared memory or TMEM when
-            // it frees them: wait (bounded, in phase order) for the copies
-            // issued and not waited for, and for every MMA commit
-            for (uint32_t i = landed; i < loaded; ++i) tc_wait(full(i % NS), (i / NS) & 1u);
-            for (uint32_t q = 0; q < NS; ++q)
-                for (uint32_t u = retired[q]; u < committed[q]; ++u) tc_wait(empty(q), u & 1u);
+            // no MMA may still read shared memory or write TMEM when they are
+            // reused or freed: wait (bounded) for each stage's last commit
+            for (uint32_t i = committed > NS ? committed - NS : 0u; i < committed; ++i)
+                tc_wait(empty(i % NS), (i / NS) & 1u);
         }
         __syncwarp();
     } else {
-        float acc_re[kTcN], acc_im[kTcN];
 #pragma unroll
-        for (uint32_t j = 0; j < kTcN; ++j) acc_re[j] = acc_im[j] = 0.f;
-        const uint32_t lane_addr = tmem + ((warp * 32u) << 16);   // this warp's 32 TMEM lanes
+        for (uint32_t j = 0; j < 64; ++j) acc_re[j] = acc_im[j] = 0.f;
+        // this warp's 32 TMEM lanes and 64 columns
+        const uint32_t addr = tmem + (((warp & 3u) * 32u) << 16) + (warp >> 2) * 64u;
         for (uint32_t b = 0; b < n_blocks; ++b) {
             const uint32_t buf = b & 1u;
             if (!s_ok) break;
@@ -540,36 +557,68 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-            for (uint32_t c0 = 0; c0 < kTcN; c0 += 8u) {
-                float vr[8], vi[8];
-                tc_ld2x8(lane_addr + buf * kTcBufCols + c0, lane_addr + buf * kTcBufCols + kTcN + c0, vr, vi);
+            for (uint32_t c0 = 0; c0 < 64; c0 += 32u) {
+                uint32_t v[64];
+                tc_ld2x32(addr + buf * T::kBufCols + c0, addr + buf * T::kBufCols + kN + c0, v);
 #pragma unroll
-                for (uint32_t j = 0; j < 8; ++j) {
-                    acc_re[c0 + j] += vr[j];
-                    acc_im[c0 + j] += vi[j];
+                for (uint32_t j = 0; j < 32; ++j) {
+                    acc_re[c0 + j] += __uint_as_float(v[j]);
+                    acc_im[c0 + j] += __uint_as_float(v[32 + j]);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty(buf)) : "memory");
         }
-        if (s_ok) {
-            const uint32_t m = mt * kTcM + warp * 32u + lane;
-            if (m < M) {
-                float2* crow = C + ((uint64_t)f * M + m) * N;
+    }
+    __syncthreads();   // no copy or MMA is left: the stages become the finished tile
+    if (warp < T::kEpilogueWarps) {
+        float4* row = reinterpret_cast<float4*>(smem + ((warp & 3u) * 32u + lane) * T::kRowBytes + (warp >> 2) * 512u);
 #pragma unroll
-                for (uint32_t j = 0; j < kTcN; ++j) {
-                    const uint32_t n = nt * kTcN + j;
-                    if (n < N) crow[n] = make_float2(acc_re[j], acc_im[j]);
+        for (uint32_t j = 0; j < 64; j += 2) row[j / 2] = make_float4(acc_re[j], acc_im[j], acc_re[j + 1], acc_im[j + 1]);
+    }
+    auto cluster_sync = [&]() {
+        if (split > 1)
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        else
+            __syncthreads();
+    };
+    cluster_sync();
+    // rows rank, rank + split, ... of the tile, the CTAs' sums added in rank
+    // order; a warp stores whole rows, two columns per lane
+    const uint32_t ok = s_ok;
+    for (uint32_t r = rank + warp * split; r < kTcM; r += (T::kEpilogueWarps + 2) * split) {
+        const uint32_t m = mt * kTcM + r;
+        if (m >= M) break;
+        float2* out = C + ((uint64_t)f * M + m) * N + (uint64_t)nt * kN;
+        for (uint32_t c = 2u * lane; c < kN; c += 64u) {
+            const uint32_t at = tc_smem(smem) + r * T::kRowBytes + c * 8u;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t q = 0; q < split; ++q) {
+                float4 x;
+                if (split > 1) {
+                    uint32_t peer;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(q));
+                    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(peer) : "memory");
+                } else {
+                    x = *reinterpret_cast<const float4*>(smem + r * T::kRowBytes + c * 8u);
                 }
+                v = q == 0 ? x : make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+            }
+            const uint32_t n = nt * kN + c;
+            if (ok && vec && n + 1 < N) {
+                *reinterpret_cast<float4*>(out + c) = v;
+            } else if (ok) {
+                if (n < N) out[c] = make_float2(v.x, v.y);
+                if (n + 1 < N) out[c + 1] = make_float2(v.z, v.w);
             }
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcTmemCols));
+    cluster_sync();   // a CTA's shared memory is read until here
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kTmemCols));
 }
-
-constexpr size_t kTcSmemBytes = kTcStages * kTcStageWords * 4 + (2 * kTcStages + 4) * 8 + 16;
 
 static uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 
@@ -580,6 +629,35 @@ static bool use_tensor_cores(int32_t mode, int64_t K, int64_t M, int64_t N) {
     if (mode == 1) return false;
     if (mode == 2) return true;
     return K >= 32 && M >= 64 && N >= 64;
+}
+
+// Tile columns and CTAs per tile of a shape: the smallest estimate of rounds
+// of CTAs on 148 SMs x 32-k blocks per CTA x time per block (128 x 128 tiles
+// take about 1.6 times as long per block as 128 x 64 ones: 40 against 28 KB
+// through L2, 768 against 384 tensor cycles per 8 k, both partly hidden),
+// plus the tile's epilogue (about four blocks' time) and the cluster's sums.
+struct TcShape {
+    uint32_t n, split;
+    uint64_t k_blocks, row_tiles, col_tiles;
+};
+
+static TcShape tc_shape(int64_t K, int64_t F, int64_t M, int64_t N) {
+    TcShape best{};
+    double least = 1e300;
+    for (uint32_t n : {128u, 64u})
+        for (uint32_t split : {1u, 2u, 4u, 8u}) {
+            TcShape s{n, split, round_up(K, kTcK) / kTcK, round_up(M, kTcM) / kTcM, round_up(N, n) / n};
+            if (split > 1 && s.k_blocks < 2 * split) continue;
+            const uint64_t ctas = (uint64_t)F * s.row_tiles * s.col_tiles * split;
+            const double rounds = (double)((ctas + 147) / 148);
+            const double cost = rounds * ((double)((s.k_blocks + split - 1) / split) + 4.0 + (split > 1 ? 1.0 : 0.0)) *
+                                (n == 128 ? 1.6 : 1.0);
+            if (cost < least) {
+                least = cost;
+                best = s;
+            }
+        }
+    return best;
 }
 
 static int cuda_fail_c(cudaError_t e, const char* what) {
@@ -620,10 +698,52 @@ int qtb_contract_sum_scratch_bytes(int64_t K, int64_t F, int64_t M, int64_t N, i
         *bytes = 16;
         return QTB_OK;
     }
-    const uint64_t Kp = round_up(K, kTcK), Mp = round_up(M, kTcM), Np = round_up(N, kTcN);
-    *bytes = 256 + (uint64_t)F * kTcPlanes * (Mp + 2 * Np) * Kp * 4;   // B planes hold two rows per column
+    const TcShape s = tc_shape(K, F, M, N);
+    // four planes of A, two of B with three rows per column
+    *bytes = 256 + (uint64_t)F * (kTcAPlanes * s.row_tiles * kTcM + kTcBPlanes * 3 * s.col_tiles * s.n) * s.k_blocks * kTcK * 4;
     return QTB_OK;
 }
+
+}  // extern "C"
+
+template <uint32_t kN>
+static cudaError_t tc_launch(const TcShape& t, const float2* A, const float2* B, float2* C, int64_t K, int64_t F,
+                             int64_t M, int64_t N, void* scratch, cudaStream_t st) {
+    using T = TcTile<kN>;
+    int* status = static_cast<int*>(scratch);
+    const uint64_t k_tiles = t.k_blocks * kTcStagesPerBlock;
+    uint32_t* Ap = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + 256);
+    uint32_t* Bp = Ap + (uint64_t)F * t.row_tiles * k_tiles * kTcAPlanes * kTcAWords;
+    const uint64_t a_blocks = (uint64_t)F * t.row_tiles * k_tiles;   // 128 rows x 2 chunks = 256 threads
+    const uint64_t b_blocks = ((uint64_t)F * t.col_tiles * k_tiles * kN * kTcChunks + 255) / 256;
+    qtb_tc_split_kernel<kN><<<(unsigned)(a_blocks + b_blocks), 256, 0, st>>>(
+        A, B, reinterpret_cast<uint4*>(Ap), reinterpret_cast<uint4*>(Bp), (uint32_t)K, (uint32_t)F, (uint32_t)M,
+        (uint32_t)N, (uint32_t)k_tiles, (uint32_t)t.row_tiles, (uint32_t)t.col_tiles, (uint32_t)a_blocks, status);
+    // per device and cheap: set on every call
+    cudaError_t e = cudaFuncSetAttribute(qtb_tc_contract_kernel<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)T::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(t.col_tiles * t.split), (unsigned)t.row_tiles, (unsigned)F);
+    cfg.blockDim = dim3(T::kThreads);
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // griddepcontrol.wait in the kernel
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = t.split;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = t.split > 1 ? 2 : 1;
+    const uint32_t vec = N % 2 == 0 && aligned16(C);
+    return cudaLaunchKernelEx(&cfg, qtb_tc_contract_kernel<kN>, (const uint32_t*)Ap, (const uint32_t*)Bp, C, (uint32_t)M,
+                              (uint32_t)N, (uint32_t)t.row_tiles, (uint32_t)t.col_tiles, (uint32_t)t.k_blocks, t.split,
+                              vec, status);
+}
+
+extern "C" {
 
 int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64_t F, int64_t M, int64_t N,
                          int32_t mode, void* scratch, size_t scratch_bytes, void* stream) {
@@ -657,29 +777,16 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
         e = cudaGetLastError();
         return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
     }
-    const uint64_t Kp = round_up(K, kTcK), Mp = round_up(M, kTcM), Np = round_up(N, kTcN);
-    if (Mp / kTcM > 65535 || F > 65535 || Np / kTcN > (1u << 31) || Kp > (1u << 30) ||
-        (uint64_t)F * (Mp / kTcM) * (Kp / kTcStageK) >= (1ull << 31) ||
-        (uint64_t)F * (Np / kTcN) * (Kp / kTcStageK) >= (1ull << 31))
+    const TcShape t = tc_shape(K, F, M, N);
+    const uint64_t k_tiles = t.k_blocks * kTcStagesPerBlock;
+    if (t.row_tiles > 65535 || F > 65535 || t.col_tiles * t.split > (1u << 30) || K > (1ll << 30) ||
+        (uint64_t)F * (t.row_tiles + t.col_tiles) * k_tiles >= (1ull << 31))
         return fail(QTB_ERR_UNSUPPORTED, "contract_sum: shape beyond the tensor-core grid");
-    e = cudaMemsetAsync(scratch, 0, 16, st);   // status word
-    if (e != cudaSuccess) return cuda_fail_c(e, "contract_sum status reset");
-    uint32_t* Ap = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + 256);
-    uint32_t* Bp = Ap + (uint64_t)F * kTcPlanes * Mp * Kp;
-    const uint32_t k_tiles = (uint32_t)(Kp / kTcStageK);
-    qtb_tc_split_kernel<<<(unsigned)(F * (Mp / kTcM) * k_tiles), 256, 0, st>>>(
-        static_cast<const float2*>(A), Ap, (uint32_t)K, (uint32_t)F, (uint32_t)M, (uint32_t)Mp, (uint32_t)Kp);
-    qtb_tc_split_b_kernel<<<(unsigned)(F * (Np / kTcN) * k_tiles), 256, 0, st>>>(
-        static_cast<const float2*>(B), Bp, (uint32_t)K, (uint32_t)F, (uint32_t)N, (uint32_t)Np, (uint32_t)Kp);
-    // per device and cheap: set on every call
-    e = cudaFuncSetAttribute(qtb_tc_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kTcSmemBytes);
-    if (e != cudaSuccess) return cuda_fail_c(e, "contract_sum smem attribute");
-    dim3 grid((unsigned)(Np / kTcN), (unsigned)(Mp / kTcM), (unsigned)F);
-    qtb_tc_contract_kernel<<<grid, kTcThreads, kTcSmemBytes, st>>>(Ap, Bp, static_cast<float2*>(C), (uint32_t)F,
-                                                                  (uint32_t)M, (uint32_t)N, (uint32_t)Mp,
-                                                                  (uint32_t)Np, (uint32_t)Kp, status);
-    e = cudaGetLastError();
+    const float2 *pa = static_cast<const float2*>(A), *pb = static_cast<const float2*>(B);
+    float2* pc = static_cast<float2*>(C);
+    e = t.n == 128 ? tc_launch<128>(t, pa, pb, pc, K, F, M, N, scratch, st)
+                   : tc_launch<64>(t, pa, pb, pc, K, F, M, N, scratch, st);
+    if (e == cudaSuccess) e = cudaGetLastError();
     return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
 }
 
