@@ -1019,63 +1019,66 @@ __global__ void __launch_bounds__(kWarpMaxThreads) qtb_warp_network_kernel(const
 
 // ----------------------------------------------------------------- K4
 // Wide networks (arenas too large for shared memory) are contracted by the
-// whole GPU at once.  Every phase of every network of a wave is cut into
-// items -- one per large op, one per run of small ops, one per run of whole
-// phases too small to split -- and every item into tiles.  Tiles whose
-// network has finished the previous phase are in a queue; CTAs take tickets
-// for its places in order and wait for their place to be filled.  The CTA
-// that finishes a phase's last tile (one counter per network and phase)
-// queues the tiles of the network's next phase, so every network advances
-// at its own pace and a CTA only waits when no tile at all is ready.
-// A ticket's place is filled by the tiles that running CTAs hold, and a CTA
-// holds a second ticket only while the place of that ticket is filled
-// already, so the scheme needs no co-residency guarantee (no cooperative
-// launch), and every wait is bounded.
+// whole GPU at once, each by a team of CTAs.  A network is a list of steps --
+// a phase, or a run of phases too small to split -- a step a list of items --
+// one per large op, one per run of small ops -- and an item is cut into
+// tiles, about one per CTA of the team.  CTAs take tickets, which name the
+// network to work on; a member of a team claims tiles of a step from the
+// step's counter, and of the next step once the step has none left, prepares
+// the tile, waits until every tile of the step before is finished (the
+// step's second counter) and contracts it.  Teams are elastic: any CTA that
+// claims does the work, so a CTA that starts late only makes its team smaller
+// until then.  A CTA only waits for tiles that were claimed before it
+// claimed its own, i.e. by CTAs that are running and that wait, if at all,
+// for an earlier step: the scheme needs no co-residency guarantee (no
+// cooperative launch), and every wait is bounded.
 struct WideNet {
     const DevNetRun* run;
     float2* term;
     uint64_t arena_off;     // complex64 elements into the wave's arenas
-    uint64_t pad;
+    uint32_t step_begin;    // its steps
+    uint32_t n_steps;
+};
+
+struct WideStep {
+    uint32_t tile_begin;    // into tile_item
+    uint32_t n_tiles;
 };
 
 struct WideItem {
-    uint64_t arena_off;     // the network's arena, complex64 elements into the wave's arenas
     uint64_t plan_off;      // bytes into the plan blobs: the network's ops (kWideOp: the op's operands)
     uint32_t a;             // the network's operands, bytes after its ops (kWideOp: the op's output)
     uint32_t begin, end;    // its ops (kWideChain: its phases; kWideOp: output variables | operands << 8 | sum << 16)
     uint32_t elem_begin;    // elements of the phase that it covers (kWideChain: the network's phases)
-    uint32_t elem_end;
-    uint32_t tile_elems;    // elements per tile
-    uint32_t done;          // counter of its phase
-    uint32_t need;          // tiles of its phase
-    uint32_t next;          // items and tiles of the network's next phase
-    uint32_t next_items;
-    uint32_t next_tiles;
-    uint32_t kind_net;      // kind | last phase << 2 | network << 3
+    uint32_t elem_end;      // (kWideChain: the first of its ops)
+    uint32_t tile_elems;    // elements per tile (kWideChain: its ops)
+    uint32_t tile_begin;    // its first tile (into tile_item)
+    uint32_t kind;
+    uint32_t in_begin;      // kWideChain: the first of its operands
+    uint32_t n_ins;         // and how many
 };
 
 constexpr uint32_t kWideOp = 0;      // one op of at least kWideChunk elements
 constexpr uint32_t kWideSmall = 1;   // a run of ops of one phase
 constexpr uint32_t kWideChain = 2;   // whole phases, one tile: the CTA's barriers separate them
+constexpr uint32_t kWideNone = 0xffffffffu;
 
 struct WideArgs {
     const WideNet* nets;
+    const WideStep* steps;
     const WideItem* items;
-    // zeroed per launch: [0] tickets taken, [1] places filled by finished
-    // phases, then the finished tiles of every network and phase
+    const uint32_t* tile_item;   // the item of every tile
+    const uint32_t* tickets;     // the network of every ticket
+    // zeroed per launch: [0] tickets taken, then per step its claimed and its
+    // finished tiles
     unsigned int* counters;
-    // the places after the first n_ready: (item + 1) << 32 | tile of the
-    // item, 0 while empty (zeroed per launch)
-    unsigned long long* queue;
-    const unsigned long long* ready;   // the first n_ready places: every network's first phase
     float2* arenas;
-    uint32_t n_tiles;
-    uint32_t n_ready;
+    uint32_t n_tickets;
     uint32_t vec;                // arenas are 16-byte aligned
 };
 
 static_assert(sizeof(WideNet) == 32, "WideNet layout");
-static_assert(sizeof(WideItem) == 64, "WideItem layout");
+static_assert(sizeof(WideItem) == 48, "WideItem layout");
 constexpr uint32_t kWideSpinLimit = 1u << 23;   // about 1 s of polling
 constexpr int kWideThreads = 256;
 constexpr int kWideCtasPerSm = 4;                       // 64 registers per thread
@@ -1083,25 +1086,16 @@ constexpr uint32_t kWideChunk = 4 * kWideThreads;       // elements of an op tha
 constexpr uint32_t kWideMaxK = 16;                      // operands of a kWideOp item
 constexpr uint32_t kWideGroup = 16;                     // chunks whose operand addresses are prepared at once
 constexpr uint32_t kWideMaxTileChunks = 64;
-constexpr uint32_t kWideSmallElems = 2;                 // elements per thread and pass of small ops
-constexpr uint32_t kWideSmallTile = kWideSmallElems * kWideThreads;
-constexpr uint32_t kWideChainElems = 512;               // largest phase of a chain
+constexpr uint32_t kWideSmallTile = kWideThreads;       // elements of small ops that a CTA contracts at once
+constexpr uint32_t kWideMaxSmallTile = 8 * kWideSmallTile;
+constexpr uint32_t kWideChainElems = kWideThreads;      // largest phase of a chain
+constexpr uint32_t kWideStage = 700;                    // 16-byte ops and operands a chain keeps in shared memory
 constexpr uint32_t kWideSmemOps = 2048;                 // ops whose first elements a tile keeps in shared memory
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-
-__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Bounded wait until *counter reaches need (acquire).  Returns false after
@@ -1232,67 +1226,90 @@ __device__ __forceinline__ void compute_elements_wide(const DevOp& op, uint32_t 
         arena[op.dst + j + e * 256u] = op.sum ? make_float2(p0[e].x + p1[e].x, p0[e].y + p1[e].y) : p0[e];
 }
 
-// Elements g0, g0 + 256, ... (kWideSmallElems of them, below g_end) of ops
-// lo .. hi - 1 of a phase, whatever their sizes: each element finds its op by
-// binary search over the ops' first elements (`first` in shared memory, or
-// null: the ops are too many) and gathers each operand's offset for itself.  The elements
-// of a thread go through every dependent load (op search, op, operand
-// descriptor, operand) together, so that their latencies overlap.
-__device__ __forceinline__ void wide_small(const DevOp* ops, uint32_t lo, uint32_t hi, uint32_t g0, uint32_t g_end,
-                                           const uint32_t* first, const DevIn* ins, const float2* table,
-                                           float2* arena) {
-    constexpr uint32_t E = kWideSmallElems;
-    uint32_t at[E], g[E];
-#pragma unroll
-    for (uint32_t i = 0; i < E; ++i) {
-        at[i] = lo;
-        g[i] = min(g0 + i * kWideThreads, g_end - 1u);
-    }
+// An element of a small op, located before the phase it reads is finished:
+// where its first four operands lie, and where it goes.
+struct WideElement {
+    uint32_t src[4];       // offset in the arena, or kSrcTable | offset in the gate table
+    uint32_t stride[4];    // of the summed variable (0: the operand lacks it)
+    uint32_t k;            // operands, 0: no element
+    uint32_t dst, op;
+    bool sum;
+};
+
+template <bool kShared>
+__device__ __forceinline__ DevIn wide_in(const DevIn* p) {
+    if constexpr (kShared) return *p;
+    else return ldg_in(p);
+}
+
+__device__ __forceinline__ void wide_operand(const DevOp& op, uint32_t j, const DevIn& d, uint32_t& src,
+                                             uint32_t& stride) {
+    const uint32_t w = op.u - op.sum;
+    src = d.src + gather_bits(j, d, (1u << w) - 1u);
+    stride = (op.sum && ((d.mask >> w) & 1u)) ? 1u << (__popc(d.mask) - 1) : 0u;
+}
+
+// Element g of ops lo .. hi - 1 of a phase (ops and ins in shared memory when
+// kShared): its op by binary search over the ops' first elements (`first` in
+// shared memory, or null), then its operands' offsets.  All of it plan data.
+template <bool kShared>
+__device__ __forceinline__ void wide_locate(WideElement& e, const DevOp* ops, uint32_t lo, uint32_t hi, uint32_t g,
+                                            const uint32_t* first, const DevIn* ins) {
+    uint32_t at = lo;
     for (uint32_t size = hi - lo; size > 1u;) {
         const uint32_t half = size >> 1;
-#pragma unroll
-        for (uint32_t i = 0; i < E; ++i)
-            if ((first ? first[at[i] - lo + half] : __ldg(&ops[at[i] + half].elem_begin)) <= g[i]) at[i] += half;
+        const uint32_t begin = kShared ? ops[at + half].elem_begin
+                               : first ? first[at - lo + half] : __ldg(&ops[at + half].elem_begin);
+        if (begin <= g) at += half;
         size -= half;
     }
-    uint32_t j[E], dst[E], uk[E];
-    const DevIn* in[E];
-    uint32_t kmax = 0;
+    const DevOp op = kShared ? ops[at] : ldg_op(ops + at);
+    const uint32_t j = g - op.elem_begin;
+    e.k = op.k;
+    e.sum = op.sum;
+    e.dst = op.dst + j;
+    e.op = at;
 #pragma unroll
-    for (uint32_t i = 0; i < E; ++i) {
-        const DevOp op = ldg_op(ops + at[i]);
-        j[i] = g[i] - op.elem_begin;
-        dst[i] = op.dst + j[i];
-        in[i] = ins + op.in_begin;
-        uk[i] = (uint32_t)op.k | (op.sum ? 0x100u : 0u) | (uint32_t)(op.u - op.sum) << 16;
-        kmax = max(kmax, (uint32_t)op.k);
-    }
-    float2 p0[E], p1[E];
+    for (uint32_t t = 0; t < 4; ++t)
+        if (t < e.k) wide_operand(op, j, wide_in<kShared>(ins + op.in_begin + t), e.src[t], e.stride[t]);
+}
+
+__device__ __forceinline__ const float2* wide_at(uint32_t src, const float2* table, const float2* arena) {
+    const float2* p = (src & kSrcTable) ? table + (src & ~kSrcTable) : arena + src;
+    __builtin_assume(__isGlobal(p));
+    return p;
+}
+
+// The element itself, in operand order.
+template <bool kShared>
+__device__ __forceinline__ void wide_contract(const WideElement& e, const DevOp* ops, const DevIn* ins,
+                                              const float2* table, float2* arena) {
+    if (e.k == 0) return;
+    float2 x0[4], x1[4];
+#pragma unroll
+    for (uint32_t t = 0; t < 4; ++t)
+        if (t < e.k) {
+            const float2* x = wide_at(e.src[t], table, arena);
+            x0[t] = x[0];
+            x1[t] = x[e.stride[t]];
+        }
+    float2 p0 = x0[0], p1 = x1[0];
+#pragma unroll
+    for (uint32_t t = 1; t < 4; ++t)
+        if (t < e.k) {
+            p0 = cmul(p0, x0[t]);
+            p1 = cmul(p1, x1[t]);
+        }
 #pragma unroll 1
-    for (uint32_t t = 0; t < kmax; ++t) {
-        float2 x0[E], x1[E];
-#pragma unroll
-        for (uint32_t i = 0; i < E; ++i)
-            if (t < (uk[i] & 0xffu)) {
-                const DevIn d = ldg_in(in[i] + t);
-                const uint32_t w = uk[i] >> 16;
-                const float2* x = ((d.src & kSrcTable) ? table + (d.src & ~kSrcTable) : arena + d.src) +
-                                  gather_bits(j[i], d, (1u << w) - 1u);
-                const bool has = (uk[i] & 0x100u) && ((d.mask >> w) & 1u);
-                x0[i] = *x;
-                x1[i] = has ? x[1u << (__popc(d.mask) - 1)] : x0[i];
-            }
-#pragma unroll
-        for (uint32_t i = 0; i < E; ++i)
-            if (t < (uk[i] & 0xffu)) {
-                p0[i] = t == 0 ? x0[i] : cmul(p0[i], x0[i]);
-                p1[i] = t == 0 ? x1[i] : cmul(p1[i], x1[i]);
-            }
+    for (uint32_t t = 4; t < e.k; ++t) {
+        const DevOp op = kShared ? ops[e.op] : ldg_op(ops + e.op);
+        uint32_t src, stride;
+        wide_operand(op, e.dst - op.dst, wide_in<kShared>(ins + op.in_begin + t), src, stride);
+        const float2* x = wide_at(src, table, arena);
+        p0 = cmul(p0, x[0]);
+        p1 = cmul(p1, x[stride]);
     }
-#pragma unroll
-    for (uint32_t i = 0; i < E; ++i)
-        if (g0 + i * kWideThreads < g_end)
-            arena[dst[i]] = (uk[i] & 0x100u) ? make_float2(p0[i].x + p1[i].x, p0[i].y + p1[i].y) : p0[i];
+    arena[e.dst] = e.sum ? make_float2(p0.x + p1.x, p0.y + p1.y) : p0;
 }
 
 // An operand of a large op: how its offset moves with the bits that are not
@@ -1434,165 +1451,216 @@ __device__ __forceinline__ void wide_chunk(const WideOperands& s, uint32_t c, ui
 struct WideShared {
     union {
         WideOperands o;                    // a large op's
-        uint32_t op_first[kWideSmemOps];   // small ops
+        uint32_t op_first[kWideSmemOps];   // small ops'
+        uint4 stage[kWideStage];           // a chain's ops and operands
     };
-    unsigned long long place;   // of the tile to run; 0: no tile left, or the wait ran out
-    uint32_t finished, first_place, last;
+    // what a tile's bookkeeping needs again after its elements lives here,
+    // not in registers
+    WideNet net;
+    uint32_t net_i;
+    uint32_t step, tile;    // the claimed tile (into tile_item); step == net.n_steps: none left
+    uint32_t tiles;         // of that step
+    int ok, last;
 };
 
-// The place of ticket t (one thread; bounded wait until it is filled).
-__device__ unsigned long long wide_place(const WideArgs& w, uint32_t t, int* status) {
-    if (t >= w.n_tiles) return 0ull;
-    if (t < w.n_ready) return w.ready[t];
-    const unsigned long long* p = w.queue + (t - w.n_ready);
-    unsigned long long v;
-    for (uint32_t it = 0; (v = ld_acquire64(p)) == 0ull;) {
-        if (++it > kWideSpinLimit) {
-            atomicOr(status, kStatusWideTimeout);
-            return 0ull;
+// Thread 0: the next tile of the team's network into s.step and s.tile, from
+// claim `c` on step s.step.
+__device__ __forceinline__ void wide_claim(WideShared& s, const WideArgs& w, uint32_t c) {
+    uint32_t step = s.step;
+    for (;;) {
+        const uint32_t at = s.net.step_begin + step;
+        const uint2 st = __ldg(reinterpret_cast<const uint2*>(w.steps + at));   // first tile, tiles
+        if (c < st.y) {
+            s.tile = st.x + c;
+            s.tiles = st.y;
+            break;
         }
-        if (it > 16) __nanosleep(64);
+        if (++step == s.net.n_steps) break;
+        c = atomicAdd(w.counters + 1 + 2 * (at + 1), 1u);
     }
-    return v;
+    s.step = step;
+}
+
+// Thread 0 waits until every tile of the step before is finished (bounded);
+// every thread returns whether they are.
+__device__ __forceinline__ bool wide_wait(WideShared& s, const WideStep* steps, unsigned int* counters, int* status) {
+    if (threadIdx.x == 0) {
+        const uint32_t at = s.net.step_begin + s.step;
+        if (s.step > 0)
+            s.ok = wait_counter(counters + 2 * at, __ldg(&steps[at - 1].n_tiles), kWideSpinLimit, status,
+                                kStatusWideTimeout);
+        __threadfence();
+    }
+    __syncthreads();
+    return s.ok != 0;
 }
 
 // A tile of small ops: a run of ops of one phase, or whole phases one after
 // another.  Out of line, so that its registers are not the large ops'.
-__device__ __noinline__ void wide_small_tile(WideShared& s, const uint4* ip, uint32_t tile, float2* arenas,
-                                             const uint4* blobs, const float2* table) {
+// Returns false when the wait ran out.
+__device__ __noinline__ bool wide_small_tile(WideShared& s, const uint4* ip, const WideStep* steps,
+                                             unsigned int* counters, float2* arenas, const uint4* blobs,
+                                             const float2* table, int* status) {
     __builtin_assume(__isShared(&s));
     const uint32_t tid = threadIdx.x;
     const uint4 i0 = __ldg(ip), i1 = __ldg(ip + 1), i2 = __ldg(ip + 2);
-    float2* arena = arenas + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
-    const char* plan = reinterpret_cast<const char*>(blobs) + ((uint64_t)i0.z | (uint64_t)i0.w << 32);
+    float2* arena = arenas + s.net.arena_off;
+    const char* plan = reinterpret_cast<const char*>(blobs) + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
     const DevOp* ops = reinterpret_cast<const DevOp*>(plan);
-    const DevIn* ins = reinterpret_cast<const DevIn*>(plan + i1.x);
-    const uint4* phases = reinterpret_cast<const uint4*>(plan) - i1.w;
-    const bool chain = (__ldg(&reinterpret_cast<const WideItem*>(ip)->kind_net) & 3u) == kWideChain;
-    const uint32_t e0 = i1.w + tile * i2.y;   // elements of the phase
-    for (uint32_t p = chain ? i1.y : 0u; p < (chain ? i1.z : 1u); ++p) {
-        uint32_t lo = i1.y, hi = i1.z, g = e0 + tid, g_end = min(e0 + i2.y, i2.x);
-        if (chain) {
-            const uint4 ph = __ldg(phases + p);   // first op, ops, elements
-            lo = ph.x;
-            hi = ph.x + ph.y;
-            g = tid;
-            g_end = ph.z;
+    const DevIn* ins = reinterpret_cast<const DevIn*>(plan + i0.z);
+    WideElement e;
+    if (i2.y == kWideSmall) {
+        const uint32_t e0 = i1.y + (s.tile - i2.x) * i1.w, g = e0 + tid;   // element of the phase
+        const uint32_t lo = i0.w, n_ops = i1.x - lo;
+        const bool staged = n_ops > 1u && n_ops <= kWideSmemOps;
+        if (staged) {
+            for (uint32_t o = tid; o < n_ops; o += kWideThreads) s.op_first[o] = __ldg(&ops[lo + o].elem_begin);
+            __syncthreads();
         }
-        const bool staged = hi - lo <= kWideSmemOps;
-        if (staged && hi - lo > 1u)
-            for (uint32_t o = tid; o < hi - lo; o += kWideThreads) s.op_first[o] = __ldg(&ops[lo + o].elem_begin);
-        __syncthreads();   // (and the phase before is written)
-        for (; g < g_end; g += kWideSmallTile)
-            wide_small(ops, lo, hi, g, g_end, staged ? s.op_first : nullptr, ins, table, arena);
-        if (chain) __syncthreads();
+        const uint32_t g_end = min(e0 + i1.w, i1.z);
+        e.k = 0;
+        if (g < g_end) wide_locate<false>(e, ops, lo, i1.x, g, staged ? s.op_first : nullptr, ins);
+        if (!wide_wait(s, steps, counters, status)) return false;
+        for (uint32_t at = g; at < g_end; at += kWideThreads) {
+            if (at != g) wide_locate<false>(e, ops, lo, i1.x, at, staged ? s.op_first : nullptr, ins);
+            wide_contract<false>(e, ops, ins, table, arena);
+        }
+        return true;
     }
+    const uint4* phases = reinterpret_cast<const uint4*>(plan) - i1.y;
+    const uint32_t n_ops = i1.w, n_ins = i2.w;
+    const bool staged = n_ops + n_ins <= kWideStage;
+    if (staged) {
+        const uint4* from = reinterpret_cast<const uint4*>(ops + i1.z);
+        for (uint32_t o = tid; o < n_ops; o += kWideThreads) s.stage[o] = __ldg(from + o);
+        from = reinterpret_cast<const uint4*>(ins + i2.z);
+        for (uint32_t o = tid; o < n_ins; o += kWideThreads) s.stage[n_ops + o] = __ldg(from + o);
+    }
+    if (!wide_wait(s, steps, counters, status)) return false;
+    const DevOp* sops = reinterpret_cast<const DevOp*>(s.stage) - i1.z;
+    const DevIn* sins = reinterpret_cast<const DevIn*>(s.stage + n_ops) - i2.z;
+    for (uint32_t p = i0.w; p < i1.x; ++p) {
+        const uint4 ph = __ldg(phases + p);   // first op, ops, elements
+        e.k = 0;
+        if (staged) {
+            if (tid < ph.z) wide_locate<true>(e, sops, ph.x, ph.x + ph.y, tid, nullptr, sins);
+            wide_contract<true>(e, sops, sins, table, arena);
+        } else {
+            if (tid < ph.z) wide_locate<false>(e, ops, ph.x, ph.x + ph.y, tid, nullptr, ins);
+            wide_contract<false>(e, ops, ins, table, arena);
+        }
+        if (p + 1u < i1.x) __syncthreads();
+    }
+    return true;
 }
 
-// Arena reads are plain loads: the queue's acquire and the barrier after it
+// Arena reads are plain loads: the wait's acquire and the barrier after it
 // order them after the other CTAs' writes, and operands that lack some of a
 // tile's element bits (an operand holds about half of them) are reused from
-// L1.  What bounds the kernel is the latency of a tile's dependent steps
-// (ticket, place, item, operand descriptors, then one round of loads per
-// operand), hence four small CTAs per SM, and the next ticket taken ahead
-// while more tiles are ready than CTAs run.  Energies of 3-regular N=256
-// p=4 and Erdos-Renyi N=400 p=3 graphs: 1030 and 1490 us with whole-GPU
-// steps (every tile waited for every network's previous phase, and thread
-// by thread for its own lookups), 422 and 505 us so.  Measured and not
-// kept: three CTAs per SM with the next operand's loads in flight (480 and
-// 635 us), every operand value loaded whether it varies or not (433 and
-// 541 us), the finishing CTA going on with its network's next phase while
-// it holds a ticket (482 and 635 us: the ticket's tile waits for it).
+// L1.  What bounds the kernel is the networks' chains of about forty phases,
+// each a barrier of its team: hence everything that does not depend on the
+// phase before -- the claim, taken while the last tile is contracted, the
+// item, the operands' offsets -- comes before the wait, and four small CTAs
+// per SM fill one another's waits.  Energies of 3-regular N=256 p=4 and
+// Erdos-Renyi N=400 p=3 graphs: 1030 and 1490 us with whole-GPU steps (every
+// tile waited for every network's previous phase, and thread by thread for
+// its own lookups), 421 and 505 us with one queue of all ready tiles (about
+// 10 us per phase to hand a network on), 381 and 493 us with teams.  Measured
+// and not kept: three CTAs per SM with the next operand's loads in flight (480
+// against 428 us and 635 against 545 us), five per SM (397 and 512 us), every
+// operand value loaded whether it varies or not (433 against 421 us and 541
+// against 505 us).
 __global__ void __launch_bounds__(kWideThreads, kWideCtasPerSm) qtb_wide_kernel(const WideArgs w, const RunArgs a) {
     __shared__ WideShared s;
     const uint32_t tid = threadIdx.x;
-    uint32_t ticket = 0;   // thread 0's
-    if (tid == 0) ticket = atomicAdd(w.counters, 1u);
-    for (;;) {
+    for (;;) {   // a ticket's network
         if (tid == 0) {
-            s.place = wide_place(w, ticket, a.status);
-            __threadfence();
+            const uint32_t t = atomicAdd(w.counters, 1u);
+            s.net_i = t < w.n_tickets ? w.tickets[t] : kWideNone;
+            if (s.net_i != kWideNone) s.net = w.nets[s.net_i];
+            s.step = kWideNone;
+            s.ok = 1;
         }
         __syncthreads();
-        const unsigned long long place = s.place;
-        if (place == 0ull) return;
-        // where more places are filled than CTAs run, the next ticket's is:
-        // taking it now hides the ticket's round trip and keeps nothing waiting
-        uint32_t next = 0xffffffffu;
-        if (tid == 0 && ticket + gridDim.x < w.n_ready + __ldcg(w.counters + 1)) next = atomicAdd(w.counters, 1u);
-        const uint4* ip = reinterpret_cast<const uint4*>(w.items + ((uint32_t)(place >> 32) - 1u));
-        const uint32_t kind = __ldg(&reinterpret_cast<const WideItem*>(ip)->kind_net) & 3u;
-        if (kind == kWideOp) {
-            const uint4 i0 = __ldg(ip), i1 = __ldg(ip + 1), i2 = __ldg(ip + 2);
-            float2* arena = w.arenas + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
-            const char* plan = reinterpret_cast<const char*>(a.blobs) + ((uint64_t)i0.z | (uint64_t)i0.w << 32);
-            const uint32_t e0 = (uint32_t)place * i2.y;   // elements of the op
-            // in groups of chunks; what a group needs is read from the item
-            // again, so that little stays in registers while chunks run
-            for (uint32_t c0 = 0;; c0 += kWideGroup) {
-                const uint32_t k = (i1.y >> 8) & 0xffu;
-                const bool sum = i1.y >> 16;
-                const uint32_t n = min((min(e0 + i2.y, i2.x) - e0) / kWideChunk - c0, kWideGroup);
-                wide_prepare(s.o, [&](uint32_t q) {
-                    const DevIn d = ldg_in(reinterpret_cast<const DevIn*>(plan) + q);
-                    // arena tensors start at multiples of four elements; a
-                    // gate table entry may start anywhere
-                    const bool table = d.src & kSrcTable;
-                    return WideSource{d, table ? a.gtable + (d.src & ~kSrcTable) : arena + d.src, w.vec && !table};
-                }, k, i1.y & 0xffu, sum, e0 + c0 * kWideChunk, n, c0 == 0u);
-                const bool last_group = c0 + kWideGroup >= (min(e0 + i2.y, i2.x) - e0) / kWideChunk;
-                float2* out = arena + i1.x + e0 + c0 * kWideChunk + 2u * tid;
-                for (uint32_t c = 0; c < n; ++c, out += kWideChunk) wide_chunk(s.o, c, k, sum, w.vec, out);
-                if (last_group) break;
-                __syncthreads();
+        if (s.net_i == kWideNone) return;
+        // a late CTA goes straight to the first step that still has tiles to claim
+        for (uint32_t i = tid; i < s.net.n_steps; i += kWideThreads) {
+            const uint32_t at = s.net.step_begin + i;
+            if (__ldcg(w.counters + 1 + 2 * at) < __ldg(&w.steps[at].n_tiles)) {
+                atomicMin(&s.step, i);
+                break;
             }
-        } else {
-            wide_small_tile(s, ip, (uint32_t)place, w.arenas, a.blobs, a.gtable);
         }
         __syncthreads();
-        // the CTA that finishes a phase queues the network's next one; after
-        // the last phase it writes the network's term, and the CTA that
-        // finishes the run's last network its energy
-        const uint4 i3 = __ldg(ip + 3);   // next phase: first item, items, tiles; kind and network
-        if (tid == 0) {
-            const uint2 count = __ldg(reinterpret_cast<const uint2*>(ip + 2) + 1);   // done, need
-            s.last = 0;
-            __threadfence();
-            s.finished = atomicAdd(w.counters + count.x, 1u) == count.y - 1u;
-            if (s.finished) {
+        if (s.step == kWideNone) continue;
+        if (tid == 0) wide_claim(s, w, atomicAdd(w.counters + 1 + 2 * (s.net.step_begin + s.step), 1u));
+        __syncthreads();
+        while (s.step < s.net.n_steps) {
+            const uint4* ip = reinterpret_cast<const uint4*>(w.items + __ldg(w.tile_item + s.tile));
+            const uint4 i2 = __ldg(ip + 2);   // first tile, kind
+            uint32_t claim = kWideNone;
+            if (i2.y == kWideOp) {
+                const uint4 i0 = __ldg(ip), i1 = __ldg(ip + 1);
+                float2* arena = w.arenas + s.net.arena_off;
+                const char* plan = reinterpret_cast<const char*>(a.blobs) + ((uint64_t)i0.x | (uint64_t)i0.y << 32);
+                const uint32_t e0 = (s.tile - i2.x) * i1.w;   // elements of the op
+                // in groups of chunks; what a group needs is read from the item
+                // again, so that little stays in registers while chunks run
+                for (uint32_t c0 = 0;; c0 += kWideGroup) {
+                    const uint32_t k = (i0.w >> 8) & 0xffu;
+                    const bool sum = i0.w >> 16;
+                    const uint32_t n = min((min(e0 + i1.w, i1.z) - e0) / kWideChunk - c0, kWideGroup);
+                    wide_prepare(s.o, [&](uint32_t q) {
+                        const DevIn d = ldg_in(reinterpret_cast<const DevIn*>(plan) + q);
+                        // arena tensors start at multiples of four elements; a
+                        // gate table entry may start anywhere
+                        const bool table = d.src & kSrcTable;
+                        return WideSource{d, table ? a.gtable + (d.src & ~kSrcTable) : arena + d.src, w.vec && !table};
+                    }, k, i0.w & 0xffu, sum, e0 + c0 * kWideChunk, n, c0 == 0u);
+                    if (c0 == 0u) {
+                        if (!wide_wait(s, w.steps, w.counters, a.status)) return;
+                        // the next claim travels while this tile is contracted
+                        if (tid == 0) claim = atomicAdd(w.counters + 1 + 2 * (s.net.step_begin + s.step), 1u);
+                    }
+                    const bool last_group = c0 + kWideGroup >= (min(e0 + i1.w, i1.z) - e0) / kWideChunk;
+                    float2* out = arena + i0.z + e0 + c0 * kWideChunk + 2u * tid;
+                    for (uint32_t c = 0; c < n; ++c, out += kWideChunk) wide_chunk(s.o, c, k, sum, w.vec, out);
+                    if (last_group) break;
+                    __syncthreads();
+                }
+            } else {
+                if (tid == 0) claim = atomicAdd(w.counters + 1 + 2 * (s.net.step_begin + s.step), 1u);
+                if (!wide_small_tile(s, ip, w.steps, w.counters, w.arenas, a.blobs, a.gtable, a.status)) return;
+            }
+            __syncthreads();
+            if (tid == 0) {
+                const uint32_t at = s.net.step_begin + s.step;
+                s.last = 0;
                 __threadfence();
-                if (!(i3.w & 4u)) {
-                    s.first_place = atomicAdd(w.counters + 1, i3.z);
-                } else {
-                    const WideNet wn = w.nets[i3.w >> 3];
-                    const uint32_t src = wn.run->result_src;
-                    *wn.term = (src & kSrcTable) ? a.gtable[src & ~kSrcTable] : __ldcg(w.arenas + wn.arena_off + src);
+                if (s.step + 1u < s.net.n_steps) {
+                    atomicAdd(w.counters + 2 + 2 * at, 1u);
+                } else if (atomicAdd(w.counters + 2 + 2 * at, 1u) == s.tiles - 1u) {
+                    // the network is done: its term, and after the run's last
+                    // network the energy
+                    __threadfence();
+                    const uint32_t src = s.net.run->result_src;
+                    *s.net.term = (src & kSrcTable) ? a.gtable[src & ~kSrcTable]
+                                                    : __ldcg(w.arenas + s.net.arena_off + src);
                     if (a.energy) {
                         __threadfence();
                         s.last = atomicAdd(a.done, 1u) == a.total_jobs - 1u;
                     }
                 }
+                wide_claim(s, w, claim);
             }
-            ticket = next != 0xffffffffu ? next : atomicAdd(w.counters, 1u);
-        }
-        __syncthreads();
-        if (s.finished && !(i3.w & 4u)) {
-            unsigned long long* q = w.queue + s.first_place;
-            for (uint32_t i = 0; i < i3.y; ++i) {
-                const uint4 n1 = __ldg(reinterpret_cast<const uint4*>(w.items + i3.x + i) + 1);
-                const uint4 n2 = __ldg(reinterpret_cast<const uint4*>(w.items + i3.x + i) + 2);
-                const bool one = n2.y == 0u;   // a chain
-                const uint32_t tiles = one ? 1u : (n2.x - n1.w + n2.y - 1u) / n2.y;
-                for (uint32_t t = tid; t < tiles; t += kWideThreads)
-                    st_release64(q + t, (unsigned long long)(i3.x + i + 1u) << 32 | t);
-                q += tiles;
+            __syncthreads();
+            if (s.last) {
+                __threadfence();
+                reduce_energy_call(a.terms, a.total_jobs, a.energy_groups, a.energy);
+                if (tid == 0) *a.done = 0u;   // ready for the next run
             }
         }
-        if (s.last) {
-            __threadfence();
-            reduce_energy_call(a.terms, a.total_jobs, a.energy_groups, a.energy);
-            if (tid == 0) *a.done = 0u;   // ready for the next run
-        }
+        __syncthreads();   // s is written by the next ticket
     }
 }
 
@@ -1785,8 +1853,8 @@ static CommonImage common_image(const qtb_plan* plan) {
 
 // One wave of wide networks: its tables live in RunCache::wide_buf.
 struct WideWave {
-    size_t nets_off, items_off, ready_off, queue_off, counters_off;   // bytes into wide_buf
-    uint32_t n_nets, n_tiles, n_ready;
+    size_t nets_off, steps_off, items_off, tiles_off, tickets_off, counters_off;   // bytes into wide_buf
+    uint32_t n_nets, n_tickets;
     int grid;
 };
 
@@ -1805,7 +1873,7 @@ struct RunCache {
     std::vector<LaunchClass> wclasses;  // warp schedule: large networks as classes + warp queue
     std::vector<WideWave> waves;        // wide networks (both schedules), run one after another
     void* wide_buf = nullptr;
-    size_t zeroed_off = 0, zeroed_bytes = 0;   // queues and counters of all waves, zeroed before a run
+    size_t zeroed_off = 0, zeroed_bytes = 0;   // counters of all waves, zeroed before a run
     size_t scratch_elems = 0;           // arenas of the largest wave, then the cluster arenas
     void* cl_jobs = nullptr;            // ClusterJob per network of moderate size (K5)
     int n_cl = 0;
@@ -2105,32 +2173,123 @@ static size_t net_need(const DevNetRun& r, size_t fixed, bool records) {
 // tables.
 constexpr size_t kWideWaveBytes = size_t(1) << 30;
 
-// The items of one wave's networks `members` (see WideItem), the places of
-// the queue that are filled from the start (the first phase of every
-// network), the tiles of the wave and its counters.  `slots`: resident CTAs,
-// which the tiles of large ops are sized for.
+// The tables of one wave's networks `members` (see WideNet ...); `slots`:
+// resident CTAs, which are shared out in teams.
 struct WideTables {
+    std::vector<WideStep> steps;
     std::vector<WideItem> items;
-    std::vector<unsigned long long> ready;
-    uint32_t n_tiles = 0, n_counters = 2;
+    std::vector<uint32_t> tile_item, tickets;
 };
 
-static uint32_t item_tiles(const WideItem& it) {
-    return it.tile_elems ? (it.elem_end - it.elem_begin + it.tile_elems - 1) / it.tile_elems : 1u;
+// How the tiles of a step are cut for a team: chunks per tile of large ops
+// and elements per tile of small ones, about one tile per member.
+struct WideCut {
+    uint64_t chunks = 0, small = 0;   // of the phase
+    uint32_t per_chunks = 1, per_small = kWideSmallTile;
+};
+
+static bool wide_large(const DevOp& op) { return op.k <= kWideMaxK && (1u << (op.u - op.sum)) >= kWideChunk; }
+
+static WideCut wide_cut(uint64_t chunks, uint64_t small, uint64_t team) {
+    WideCut c;
+    c.chunks = chunks;
+    c.small = small;
+    auto per = [&](uint64_t n, uint64_t most) {
+        return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(most, (n + team - 1) / team));
+    };
+    c.per_chunks = per(chunks, kWideMaxTileChunks);
+    c.per_small = kWideSmallTile * per((small + kWideSmallTile - 1) / kWideSmallTile, kWideMaxSmallTile / kWideSmallTile);
+    return c;
 }
 
-static WideTables wave_tables(const qtb_plan* plan, const std::vector<int32_t>& members,
-                              const std::vector<uint64_t>& arena_off, uint64_t slots) {
-    auto large = [](const DevOp& op) { return op.k <= kWideMaxK && (1u << (op.u - op.sum)) >= kWideChunk; };
-    // elements of large ops per phase index, over all networks
-    std::vector<uint64_t> op_elems;
-    for (int32_t m : members) {
-        const Network& n = plan->nets[m];
-        op_elems.resize(std::max(op_elems.size(), n.phases.size()), 0);
-        for (size_t ph = 0; ph < n.phases.size(); ++ph)
-            for (uint32_t o = n.phases[ph].op_first; o < n.phases[ph].op_first + n.phases[ph].op_count; ++o)
-                if (large(n.ops[o])) op_elems[ph] += 1ull << (n.ops[o].u - n.ops[o].sum);
+// CTAs per network: the fewest that finish every network within the least
+// common time that `slots` CTAs allow, by a model of the times measured per
+// tile: 8 us (claim, set-up, wait, finish, and waiting for the rest of the
+// team), (0.6 + 0.4 k) us per chunk of an op of k operands, 2.5 us per 256
+// elements of small ops, 0.8 us per phase of a chain (3 or 5.5 us per tile in
+// its place: 379 and 509 us on the two graphs at qtb_wide_kernel, 8 us 382 and
+// 492 us).
+static std::vector<uint32_t> wide_teams(const qtb_plan* plan, const std::vector<int32_t>& members, uint64_t slots) {
+    constexpr double kTileUs = 8.0, kSmallUs = 2.5, kChainUs = 0.8;
+    struct Load {
+        uint64_t chunks, small;
+        double chunk_us;   // all chunks
+    };
+    std::vector<std::vector<Load>> loads(members.size());
+    for (size_t k = 0; k < members.size(); ++k) {
+        const Network& n = plan->nets[members[k]];
+        for (const DevPhase& p : n.phases) {
+            Load l{0, 0, 0.0};
+            if (p.total_elems > kWideChainElems)
+                for (uint32_t o = p.op_first; o < p.op_first + p.op_count; ++o) {
+                    const uint64_t elems = 1ull << (n.ops[o].u - n.ops[o].sum);
+                    if (wide_large(n.ops[o])) {
+                        l.chunks += elems / kWideChunk;
+                        l.chunk_us += (0.6 + 0.4 * n.ops[o].k) * (double)(elems / kWideChunk);
+                    } else {
+                        l.small += elems;
+                    }
+                }
+            loads[k].push_back(l);
+        }
     }
+    auto time = [&](size_t k, uint64_t team) {
+        double t = 0.0;
+        for (const Load& l : loads[k]) {
+            if (l.chunks + l.small == 0) {
+                t += kChainUs;
+                continue;
+            }
+            const WideCut c = wide_cut(l.chunks, l.small, team);
+            const double a = (double)((l.chunks + c.per_chunks - 1) / c.per_chunks);
+            const double b = (double)((l.small + c.per_small - 1) / c.per_small);
+            const double ta = l.chunks ? kTileUs + l.chunk_us / (double)l.chunks * c.per_chunks : 0.0;
+            const double tb = l.small ? kTileUs + kSmallUs * c.per_small / kWideSmallTile : 0.0;
+            t += std::max(std::max(ta, tb), (a * ta + b * tb) / (double)team);
+        }
+        return t;
+    };
+    auto team_for = [&](size_t k, double limit) -> uint64_t {   // fewest CTAs within `limit`, 0: none
+        uint64_t hi = 1;
+        while (hi < slots && time(k, hi) > limit) hi *= 2;
+        hi = std::min(hi, slots);
+        if (time(k, hi) > limit) return 0;
+        uint64_t lo = 1;
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (time(k, mid) <= limit) hi = mid;
+            else lo = mid + 1;
+        }
+        return lo;
+    };
+    std::vector<uint32_t> teams(members.size(), 1);
+    double lo = 0.0, hi = 0.0;
+    for (size_t k = 0; k < members.size(); ++k) {
+        lo = std::max(lo, time(k, slots));
+        hi = std::max(hi, time(k, 1));
+    }
+    for (int it = 0; it < 24 && hi > lo; ++it) {
+        const double mid = it == 0 ? lo : 0.5 * (lo + hi);
+        uint64_t sum = 0;
+        std::vector<uint32_t> t(members.size());
+        for (size_t k = 0; k < members.size() && sum <= slots; ++k) {
+            const uint64_t g = team_for(k, mid);
+            sum += g ? g : slots + 1;
+            t[k] = (uint32_t)g;
+        }
+        if (sum <= slots) {
+            teams = t;
+            hi = mid;
+        } else {
+            lo = mid;
+        }
+    }
+    return teams;
+}
+
+static WideTables wave_tables(const qtb_plan* plan, const std::vector<int32_t>& members, uint64_t slots,
+                              std::vector<WideNet>* nets) {
+    const std::vector<uint32_t> teams = wide_teams(plan, members, slots);
     WideTables out;
     for (size_t k = 0; k < members.size(); ++k) {
         const Network& n = plan->nets[members[k]];
@@ -2138,78 +2297,82 @@ static WideTables wave_tables(const qtb_plan* plan, const std::vector<int32_t>& 
         const uint32_t np = (uint32_t)n.phases.size();
         const uint64_t blob = 16 * (uint64_t)run.blob_off16;
         WideItem base{};
-        base.arena_off = arena_off[k];
         base.plan_off = blob + np * sizeof(DevPhase);
         base.a = run.ins_off - np * (uint32_t)sizeof(DevPhase);
-        base.kind_net = (uint32_t)k << 3;
-        size_t prev_begin = 0, prev_end = 0;   // the items of the phase before
+        (*nets)[k].step_begin = (uint32_t)out.steps.size();
         uint32_t ph = 0;
         do {
             uint32_t end = ph;
             while (end < np && n.phases[end].total_elems <= kWideChainElems) ++end;
-            const size_t first = out.items.size();
-            base.done = out.n_counters++;
+            WideStep st{(uint32_t)out.tile_item.size(), 0};
+            auto add = [&](WideItem it, uint32_t tiles) {
+                it.tile_begin = (uint32_t)out.tile_item.size();
+                out.tile_item.insert(out.tile_item.end(), tiles, (uint32_t)out.items.size());
+                out.items.push_back(it);
+            };
             if (end > ph || np == 0) {
                 // np == 0: the result is a gate-table scalar, and an empty chain writes the term
                 WideItem it = base;
-                it.kind_net |= kWideChain;
+                it.kind = kWideChain;
                 it.begin = ph;
                 it.end = end;
                 it.elem_begin = np;
-                out.items.push_back(it);
+                if (end > ph) {
+                    const DevPhase &p0 = n.phases[ph], &p1 = n.phases[end - 1];
+                    const DevOp &first = n.ops[p0.op_first], &last = n.ops[p1.op_first + p1.op_count - 1];
+                    it.elem_end = p0.op_first;
+                    it.tile_elems = p1.op_first + p1.op_count - p0.op_first;
+                    it.in_begin = first.in_begin;
+                    it.n_ins = last.in_begin + last.k - first.in_begin;
+                }
+                add(it, 1);
             } else {
                 end = ph + 1;
                 const DevPhase& p = n.phases[ph];
                 const uint32_t o_end = p.op_first + p.op_count;
-                // about one tile per resident CTA over the networks' phases
-                // of this index: larger tiles spread a tile's set-up over
-                // more chunks, and networks at other phases fill the rest
-                const uint32_t chunks = (uint32_t)std::max<uint64_t>(
-                    1, std::min<uint64_t>(kWideMaxTileChunks, op_elems[ph] / (slots * kWideChunk)));
+                uint64_t op_chunks = 0;
+                for (uint32_t o = p.op_first; o < o_end; ++o)
+                    if (wide_large(n.ops[o])) op_chunks += (1u << (n.ops[o].u - n.ops[o].sum)) / kWideChunk;
+                const WideCut cut = wide_cut(op_chunks, p.total_elems - op_chunks * kWideChunk, teams[k]);
                 for (uint32_t o = p.op_first; o < o_end;) {
                     uint32_t q = o + 1;
                     WideItem it = base;
-                    if (large(n.ops[o])) {
+                    if (wide_large(n.ops[o])) {
                         const DevOp& op = n.ops[o];
-                        it.kind_net |= kWideOp;
+                        it.kind = kWideOp;
                         it.plan_off = blob + run.ins_off + op.in_begin * sizeof(DevIn);
                         it.a = op.dst;
                         it.begin = (uint32_t)(op.u - op.sum) | (uint32_t)op.k << 8 | (uint32_t)op.sum << 16;
                         it.elem_end = 1u << (op.u - op.sum);
-                        it.tile_elems = chunks * kWideChunk;
+                        it.tile_elems = cut.per_chunks * kWideChunk;
                     } else {
-                        while (q < o_end && !large(n.ops[q])) ++q;
-                        it.kind_net |= kWideSmall;
+                        while (q < o_end && !wide_large(n.ops[q])) ++q;
+                        it.kind = kWideSmall;
                         it.begin = o;
                         it.end = q;
                         it.elem_begin = n.ops[o].elem_begin;
                         it.elem_end = q < o_end ? n.ops[q].elem_begin : p.total_elems;
-                        it.tile_elems = kWideSmallTile;
+                        it.tile_elems = cut.per_small;
                     }
-                    out.items.push_back(it);
+                    add(it, (it.elem_end - it.elem_begin + it.tile_elems - 1) / it.tile_elems);
                     o = q;
                 }
             }
-            uint32_t tiles = 0;
-            for (size_t i = first; i < out.items.size(); ++i) tiles += item_tiles(out.items[i]);
-            for (size_t i = first; i < out.items.size(); ++i) {
-                out.items[i].need = tiles;
-                if (end == np) out.items[i].kind_net |= 4u;
-            }
-            for (size_t i = prev_begin; i < prev_end; ++i) {
-                out.items[i].next = (uint32_t)first;
-                out.items[i].next_items = (uint32_t)(out.items.size() - first);
-                out.items[i].next_tiles = tiles;
-            }
-            if (prev_end == 0)
-                for (size_t i = first; i < out.items.size(); ++i)
-                    for (uint32_t t = 0; t < item_tiles(out.items[i]); ++t)
-                        out.ready.push_back((unsigned long long)(i + 1) << 32 | t);
-            out.n_tiles += tiles;
-            prev_begin = first;
-            prev_end = out.items.size();
+            st.n_tiles = (uint32_t)out.tile_item.size() - st.tile_begin;
+            out.steps.push_back(st);
             ph = end;
         } while (ph < np);
+        (*nets)[k].n_steps = (uint32_t)out.steps.size() - (*nets)[k].step_begin;
+    }
+    // one CTA for every network first, then the teams' second CTAs, ...: CTAs
+    // that start late leave no network without one
+    for (uint32_t round = 0, more = 1; more; ++round) {
+        more = 0;
+        for (size_t k = 0; k < members.size(); ++k)
+            if (teams[k] > round) {
+                out.tickets.push_back((uint32_t)k);
+                more = 1;
+            }
     }
     return out;
 }
@@ -2249,22 +2412,19 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
         rc->scratch_elems = std::max(rc->scratch_elems, elems);
         if (device) {
             const std::vector<int32_t> members(wide.begin() + pos, wide.begin() + end);
-            std::vector<uint64_t> offs;
             std::vector<WideNet> wn(members.size());
             size_t off = 0;
             for (size_t k = 0; k < members.size(); ++k) {
                 wn[k].run = runs + members[k];
                 wn[k].term = terms + (members[k] - first);
                 wn[k].arena_off = off;
-                offs.push_back(off);
                 off += arena_of(members[k]);
             }
-            WideTables tb = wave_tables(plan, members, offs, slots);
+            WideTables tb = wave_tables(plan, members, slots, &wn);
             WideWave wv{};
             wv.n_nets = (uint32_t)members.size();
-            wv.n_tiles = tb.n_tiles;
-            wv.n_ready = (uint32_t)tb.ready.size();
-            wv.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(wv.n_tiles, slots));
+            wv.n_tickets = (uint32_t)tb.tickets.size();
+            wv.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(wv.n_tickets, slots));
             rc->waves.push_back(wv);
             nets.push_back(std::move(wn));
             tables.push_back(std::move(tb));
@@ -2274,36 +2434,37 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
         pos = end;
     }
     if (!device) return QTB_OK;   // sizes only (qtb_plan_scratch_bytes)
-    // device buffer: per wave [nets][items][ready], 256-byte aligned, then
-    // per wave [queue][counters], which are zeroed before a run
+    // device buffer: per wave the tables, 256-byte aligned, then the waves'
+    // counters, which are zeroed before a run
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     size_t bytes = 0;
+    auto place = [&](size_t* off, size_t n) {
+        *off = bytes;
+        bytes = align(bytes + n);
+    };
     for (size_t v = 0; v < rc->waves.size(); ++v) {
         WideWave& wv = rc->waves[v];
-        wv.nets_off = bytes;
-        bytes = align(bytes + nets[v].size() * sizeof(WideNet));
-        wv.items_off = bytes;
-        bytes = align(bytes + tables[v].items.size() * sizeof(WideItem));
-        wv.ready_off = bytes;
-        bytes = align(bytes + tables[v].ready.size() * sizeof(unsigned long long));
+        place(&wv.nets_off, nets[v].size() * sizeof(WideNet));
+        place(&wv.steps_off, tables[v].steps.size() * sizeof(WideStep));
+        place(&wv.items_off, tables[v].items.size() * sizeof(WideItem));
+        place(&wv.tiles_off, tables[v].tile_item.size() * sizeof(uint32_t));
+        place(&wv.tickets_off, tables[v].tickets.size() * sizeof(uint32_t));
     }
-    const size_t zeroed = bytes;
+    rc->zeroed_off = bytes;
     for (size_t v = 0; v < rc->waves.size(); ++v) {
-        WideWave& wv = rc->waves[v];
-        wv.queue_off = bytes;
-        bytes += (size_t)(wv.n_tiles - wv.n_ready) * sizeof(unsigned long long);
-        wv.counters_off = bytes;
-        bytes += ((size_t)tables[v].n_counters * sizeof(unsigned int) + 7) & ~size_t(7);
+        rc->waves[v].counters_off = bytes;
+        bytes += (1 + 2 * tables[v].steps.size()) * sizeof(unsigned int);
     }
-    rc->zeroed_off = zeroed;
-    rc->zeroed_bytes = bytes - zeroed;
-    std::vector<uint8_t> image(zeroed, 0);
+    rc->zeroed_bytes = bytes - rc->zeroed_off;
+    std::vector<uint8_t> image(rc->zeroed_off, 0);
+    auto put = [&](size_t off, const auto& v) { std::memcpy(image.data() + off, v.data(), v.size() * sizeof(v[0])); };
     for (size_t v = 0; v < rc->waves.size(); ++v) {
         const WideWave& wv = rc->waves[v];
-        std::memcpy(image.data() + wv.nets_off, nets[v].data(), nets[v].size() * sizeof(WideNet));
-        std::memcpy(image.data() + wv.items_off, tables[v].items.data(), tables[v].items.size() * sizeof(WideItem));
-        std::memcpy(image.data() + wv.ready_off, tables[v].ready.data(),
-                    tables[v].ready.size() * sizeof(unsigned long long));
+        put(wv.nets_off, nets[v]);
+        put(wv.steps_off, tables[v].steps);
+        put(wv.items_off, tables[v].items);
+        put(wv.tiles_off, tables[v].tile_item);
+        put(wv.tickets_off, tables[v].tickets);
     }
     QTB_CUDA(cudaMalloc(&rc->wide_buf, bytes));
     QTB_CUDA(cudaMemcpy(rc->wide_buf, image.data(), image.size(), cudaMemcpyHostToDevice));
@@ -2703,13 +2864,13 @@ static int launch_waves(const RunCache* rc, const RunArgs& base, void* scratch_d
     for (const WideWave& wv : rc->waves) {
         WideArgs w{};
         w.nets = reinterpret_cast<const WideNet*>(buf + wv.nets_off);
+        w.steps = reinterpret_cast<const WideStep*>(buf + wv.steps_off);
         w.items = reinterpret_cast<const WideItem*>(buf + wv.items_off);
-        w.queue = reinterpret_cast<unsigned long long*>(buf + wv.queue_off);
-        w.ready = reinterpret_cast<const unsigned long long*>(buf + wv.ready_off);
+        w.tile_item = reinterpret_cast<const uint32_t*>(buf + wv.tiles_off);
+        w.tickets = reinterpret_cast<const uint32_t*>(buf + wv.tickets_off);
         w.counters = reinterpret_cast<unsigned int*>(buf + wv.counters_off);
         w.arenas = static_cast<float2*>(scratch_dev);
-        w.n_tiles = wv.n_tiles;
-        w.n_ready = wv.n_ready;
+        w.n_tickets = wv.n_tickets;
         w.vec = reinterpret_cast<uintptr_t>(scratch_dev) % 16 == 0;
         qtb_wide_kernel<<<wv.grid, kWideThreads, 0, st>>>(w, base);
         QTB_CUDA(cudaGetLastError());
