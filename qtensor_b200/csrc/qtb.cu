@@ -253,6 +253,7 @@ struct RunArgs {
     const uint4* blobs;           // network blobs
     const uint4* common;          // [DevEntry x n_entries, padded to 16 B][DevTerm ...]
     uint32_t common_bytes;        // multiple of 16
+    uint32_t n_params;
     uint32_t n_entries;
     uint32_t terms_off;           // byte offset of the DevTerm array in common
     uint32_t table_elems;
@@ -342,39 +343,73 @@ __device__ __forceinline__ void neumaier_add(double& sum, double& comp, double x
     sum = t;
 }
 
-// Compensated fp64 sum of Re(terms) by one warp (all 32 lanes call it) in
-// a fixed order -- lane l sums terms l, l + 32, ..., then a butterfly --
-// then energy = (n_groups - sum) / 2.  The order does not depend on the
-// launch shape, so every schedule gives the same energy for the same terms.
-__device__ void reduce_energy_warp(const float2* terms, uint32_t n, double n_groups, double* energy) {
-    constexpr uint32_t kBatch = 16;   // loads in flight per lane: one L2 round trip per 16 terms
-    const uint32_t lane = threadIdx.x & 31u;
+// Compensated fp64 sum of Re(terms), then energy = (n_groups - sum) / 2.
+// The order is fixed, whatever the launch shape, so that every schedule
+// gives the same energy for the same terms: kSumLanes running sums (sum v of
+// terms v, v + kSumLanes, ...), a butterfly over each 32 of them, then the
+// groups of 32 in order.  One warp's running sums over all terms took 5.6 of
+// the 38 us of N=1000 p=3 (3.4 of 9.7 us for 30 terms, mostly a system-wide
+// fence that the end of the kernel makes needless); so 3.6 us and 1.4 us.
+constexpr uint32_t kSumLanes = 128, kSumGroups = kSumLanes / 32;
+
+// (sum, compensation) of group g of 32 running sums, in every lane of a warp.
+__device__ __forceinline__ double2 reduce_group(const float2* terms, uint32_t n, uint32_t g) {
+    constexpr uint32_t kBatch = 12;   // loads in flight per lane
     double s = 0.0, c = 0.0;
-    for (uint32_t base = lane; base < n; base += 32u * kBatch) {
+    for (uint32_t base = g * 32u + (threadIdx.x & 31u); base < n; base += kSumLanes * kBatch) {
         float x[kBatch];
 #pragma unroll
-        for (uint32_t j = 0; j < kBatch; ++j) x[j] = base + 32u * j < n ? __ldcg(&terms[base + 32u * j].x) : 0.f;
+        for (uint32_t j = 0; j < kBatch; ++j)
+            x[j] = base + kSumLanes * j < n ? __ldcg(&terms[base + kSumLanes * j].x) : 0.f;
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j)
-            if (base + 32u * j < n) neumaier_add(s, c, (double)x[j]);
+            if (base + kSumLanes * j < n) neumaier_add(s, c, (double)x[j]);
     }
     for (int off = 16; off > 0; off >>= 1) {
         const double os = __shfl_xor_sync(0xffffffffu, s, off);
         const double oc = __shfl_xor_sync(0xffffffffu, c, off);
         neumaier_add(s, c, os);
-        neumaier_add(s, c, oc);
+        c += oc;
     }
-    if (lane == 0) {
-        *energy = (n_groups - (s + c)) * 0.5;
-        // the energy may live in mapped host memory (a caller's pinned
-        // buffer), read by the host once the kernel is done
-        __threadfence_system();
-    }
+    return make_double2(s, c);
 }
 
-// The same by a whole CTA: its first warp sums, the others wait.
+__device__ __forceinline__ void reduce_finish(const double2 (&group)[kSumGroups], double n_groups, double* energy) {
+    double s = group[0].x, c = group[0].y;
+#pragma unroll
+    for (uint32_t g = 1; g < kSumGroups; ++g) {
+        neumaier_add(s, c, group[g].x);
+        c += group[g].y;
+    }
+    // the energy may live in mapped host memory (a caller's pinned buffer):
+    // the end of the kernel makes it visible there
+    *energy = (n_groups - (s + c)) * 0.5;
+}
+
+// By one warp (all 32 lanes call it).
+__device__ void reduce_energy_warp(const float2* terms, uint32_t n, double n_groups, double* energy) {
+    double2 group[kSumGroups];
+#pragma unroll
+    for (uint32_t g = 0; g < kSumGroups; ++g) group[g] = reduce_group(terms, n, g);
+    if ((threadIdx.x & 31u) == 0) reduce_finish(group, n_groups, energy);
+}
+
+// By a whole CTA of at least one warp (every thread calls it): its warps
+// share the groups.
 __device__ void reduce_energy(const float2* terms, uint32_t n, double n_groups, double* energy) {
-    if (threadIdx.x < 32) reduce_energy_warp(terms, n, n_groups, energy);
+    __shared__ double2 s_group[kSumGroups];
+    const uint32_t warps = blockDim.x >> 5;
+    for (uint32_t g = threadIdx.x >> 5; g < kSumGroups; g += warps) {
+        const double2 v = reduce_group(terms, n, g);
+        if ((threadIdx.x & 31u) == 0) s_group[g] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double2 group[kSumGroups];
+#pragma unroll
+        for (uint32_t g = 0; g < kSumGroups; ++g) group[g] = s_group[g];
+        reduce_finish(group, n_groups, energy);
+    }
     __syncthreads();
 }
 
@@ -540,33 +575,62 @@ __device__ __forceinline__ void l2_prefetch_part(const void* p, uint32_t bytes, 
                  : "memory");
 }
 
-// Header of phase p of a network's records (zero elements past the last).
-struct RecHead {
-    const uint32_t* rows;   // payload: row r of element g at rows[r * total + g]
-    uint32_t total;
-    uint32_t kmax;
+// Phase headers a CTA stages in shared memory for a network with records
+// (networks with more phases read the rest from global memory).
+constexpr uint32_t kRecHeadSmem = 64;
+
+// Header of phase p: x = payload offset (words), y = elements | (largest
+// operand count) << 24; zero elements past the last.
+struct RecHeads {
+    const uint2* global;
+    const uint2* shared;
+    uint32_t n;
+    __device__ __forceinline__ uint2 operator()(uint32_t p) const {
+        return p >= n ? make_uint2(0u, 0u) : n <= kRecHeadSmem ? shared[p] : __ldg(global + p);
+    }
 };
 
-__device__ __forceinline__ RecHead rec_head(const uint32_t* rec, uint32_t p, uint32_t n_phases) {
-    if (p >= n_phases) return RecHead{rec, 0u, 0u};
-    const uint2 h = __ldg(reinterpret_cast<const uint2*>(rec) + p);
-    return RecHead{rec + h.x, h.y & 0xffffffu, h.y >> 24};
+// What a thread loads of a network's records as soon as the network is
+// located, before the gate table is built: the header that it stages and, of
+// a compact-record network, its record of phase 0.  Those follow the headers
+// (rounded up to 16 bytes); the load stays inside the network's records, and
+// the record is used only if the thread has an element in phase 0.
+struct RecStart {
+    uint2 head;
+    uint4 first;
+};
+
+__device__ __forceinline__ RecStart rec_start(const DevNetRun& net, const uint32_t* __restrict__ rec) {
+    const uint32_t tid = threadIdx.x, np = net.n_phases, first_word = (2u * np + 3u) & ~3u;
+    RecStart s;
+    s.head = tid < np ? __ldg(reinterpret_cast<const uint2*>(rec) + tid) : make_uint2(0u, 0u);
+    s.first = net.rec_format == kRecCompact && first_word + 4u * (tid + 1u) <= net.rec_words
+                  ? __ldg(reinterpret_cast<const uint4*>(rec + first_word) + tid)
+                  : make_uint4(0u, 0u, 0u, 0u);
+    return s;
 }
 
-// The record words of element g (zeros past the phase or the phase's rows).
-__device__ __forceinline__ void rec_load(const RecHead& h, uint32_t g, uint32_t (&w)[kRecMaxK + 1]) {
-#pragma unroll
-    for (uint32_t t = 0; t <= kRecMaxK; ++t)
-        w[t] = (g < h.total && t <= h.kmax) ? __ldg(h.rows + (size_t)t * h.total + g) : 0u;
+// Stages the headers of a network; a barrier is passed.
+__device__ __forceinline__ RecHeads rec_heads(const uint32_t* __restrict__ rec, uint32_t n_phases, uint2 mine,
+                                              uint2* __restrict__ s_head) {
+    const RecHeads h{reinterpret_cast<const uint2*>(rec), s_head, n_phases};
+    if (n_phases <= kRecHeadSmem) {
+        if (threadIdx.x < n_phases) s_head[threadIdx.x] = mine;
+        for (uint32_t i = threadIdx.x + blockDim.x; i < n_phases; i += blockDim.x) s_head[i] = __ldg(h.global + i);
+    }
+    __syncthreads();
+    return h;
 }
 
-// One output element from its record: the same products, in the same
-// operand order, as compute_element.
-__device__ __forceinline__ void rec_element(const uint32_t (&w)[kRecMaxK + 1], float2* __restrict__ S) {
+// One output element from the words of its record (row 0, then one per
+// operand, kWords of them): the same products, in the same operand order, as
+// compute_element.
+template <uint32_t kWords>
+__device__ __forceinline__ void rec_element(const uint32_t (&w)[kWords], float2* __restrict__ S) {
     const uint32_t d = w[0], k = (d >> 16) & 0xffu;
     float2 p0 = S[w[1] & 0xffffu], p1 = S[w[1] >> 16];
 #pragma unroll
-    for (uint32_t t = 2; t <= kRecMaxK; ++t)
+    for (uint32_t t = 2; t < kWords; ++t)
         if (t <= k) {
             p0 = cmul(p0, S[w[t] & 0xffffu]);
             p1 = cmul(p1, S[w[t] >> 16]);
@@ -574,38 +638,76 @@ __device__ __forceinline__ void rec_element(const uint32_t (&w)[kRecMaxK + 1], f
     S[d & 0xffffu] = (d >> 24) ? make_float2(p0.x + p1.x, p0.y + p1.y) : p0;
 }
 
-// The phases of one network from its element records, S the shared window
-// [gate table][arena].  Each thread's record of its first element of the
-// next phase, and the header of the phase after, are loaded while the
-// current phase computes, so the loads from L2 overlap the phase and its
-// barrier instead of starting every phase.  Same phase split as
-// contract_network: phases of more than 32 elements on every thread with
+// Elements g, g + blockDim.x, ... of a phase whose ops have at most
+// kWords - 1 operands, kBatch records loaded before the first is used.
+template <uint32_t kWords, uint32_t kBatch>
+__device__ __forceinline__ void rec_rounds(const uint32_t* __restrict__ rows, uint32_t total, uint32_t kmax, uint32_t g,
+                                           float2* __restrict__ S) {
+    for (; g < total; g += kBatch * blockDim.x) {
+        uint32_t w[kBatch][kWords];
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i) {
+            const uint32_t e = min(g + i * blockDim.x, total - 1u);
+#pragma unroll
+            for (uint32_t t = 0; t < kWords; ++t) w[i][t] = t <= kmax ? __ldg(rows + (size_t)t * total + e) : 0u;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i)
+            if (g + i * blockDim.x < total) rec_element(w[i], S);
+    }
+}
+
+// The phases of one network from its wide-format element records, S the
+// shared window [gate table][arena].  A thread's record of its first element
+// is loaded two phases ahead (its first kRecAhead words: phases of more
+// operands load theirs when they start), so that the loads from L2 overlap
+// two phases and their barriers; with one phase ahead and the headers loaded
+// in turn, a phase of few elements took 0.42-0.70 us, so 0.35-0.50 us (the
+// widest N=100 p=3 network, 512 threads: 23.5 -> 20.8 us; the whole energy 50
+// -> 43.5 us with what follows and precedes it).  Same phase split
+// as contract_network: phases of more than 32 elements on every thread with
 // block barriers, the tail on warp 0 with warp barriers.
-__device__ float2 contract_records(const DevNetRun& net, const uint32_t* __restrict__ rec,
-                                   float2* __restrict__ S, const float2* __restrict__ arena) {
-    const uint32_t tid = threadIdx.x;
-    RecHead h = rec_head(rec, 0, net.n_phases);
-    RecHead h1 = rec_head(rec, 1, net.n_phases);
-    uint32_t cur[kRecMaxK + 1];
-    rec_load(h, tid, cur);
-    for (uint32_t p = 0; p < net.n_phases; ++p) {
-        const bool tail = p >= net.tail_start;
-        if (tail && tid >= 32) break;
-        uint32_t nxt[kRecMaxK + 1];
-        rec_load(h1, tid, nxt);
-        const RecHead h2 = rec_head(rec, p + 2, net.n_phases);
-        if (tid < h.total) rec_element(cur, S);
-        for (uint32_t g = tid + blockDim.x; g < h.total; g += blockDim.x) {
-            uint32_t w[kRecMaxK + 1];
-            rec_load(h, g, w);
-            rec_element(w, S);
+constexpr uint32_t kRecAhead = 6;
+
+__device__ float2 contract_records(const DevNetRun& net, const uint32_t* __restrict__ rec, float2* __restrict__ S,
+                                   const float2* __restrict__ arena, uint2* __restrict__ s_head, const RecStart& start) {
+    const uint32_t tid = threadIdx.x, np = net.n_phases;
+    const RecHeads head = rec_heads(rec, np, start.head, s_head);
+    struct Ahead {
+        uint2 h;
+        uint32_t w[kRecAhead];
+    };
+    auto first = [&](uint32_t p) {
+        Ahead a;
+        a.h = head(p);
+        const uint32_t total = a.h.y & 0xffffffu, kmax = a.h.y >> 24;
+#pragma unroll
+        for (uint32_t t = 0; t < kRecAhead; ++t)
+            a.w[t] = tid < total && t <= kmax ? __ldg(rec + a.h.x + (size_t)t * total + tid) : 0u;
+        return a;
+    };
+    auto phase = [&](uint32_t q, const Ahead& cur, Ahead& ahead) -> bool {
+        if (q >= np) return false;
+        const bool tail = q >= net.tail_start;
+        if (tail && tid >= 32) return false;
+        ahead = first(q + 2);
+        const uint32_t total = cur.h.y & 0xffffffu, kmax = cur.h.y >> 24;
+        const uint32_t* rows = rec + cur.h.x;
+        if (kmax < kRecAhead) {
+            if (tid < total) rec_element(cur.w, S);
+            if (tid + blockDim.x < total) rec_rounds<kRecAhead, 2>(rows, total, kmax, tid + blockDim.x, S);
+        } else {
+            rec_rounds<kRecMaxK + 1, 1>(rows, total, kmax, tid, S);
         }
         if (tail) __syncwarp();
         else __syncthreads();
-        h = h1;
-        h1 = h2;
-#pragma unroll
-        for (uint32_t t = 0; t <= kRecMaxK; ++t) cur[t] = nxt[t];
+        return true;
+    };
+    Ahead ra = first(0), rb = first(1), rc;
+    for (uint32_t p = 0;; p += 3) {
+        if (!phase(p, ra, rc)) break;
+        if (!phase(p + 1, rb, ra)) break;
+        if (!phase(p + 2, rc, rb)) break;
     }
     float2 result = make_float2(0.f, 0.f);
     if (tid == 0)
@@ -641,10 +743,6 @@ __device__ __forceinline__ void rec_element_compact(const uint4 r, float2* __res
     S[h & 0xfffu] = (h >> 15) ? make_float2(p0.x + p1.x, p0.y + p1.y) : p0;
 }
 
-// Phase headers a CTA stages in shared memory for a compact-record network
-// (networks with more phases read the rest from global memory).
-constexpr uint32_t kRecHeadSmem = 64;
-
 // The phases of one network from its compact records.  The phase headers
 // are staged in shared memory; each thread's record of its first element
 // in the next three phases is in flight while the current phase computes,
@@ -652,24 +750,10 @@ constexpr uint32_t kRecHeadSmem = 64;
 // phase split as contract_network.
 __device__ float2 contract_records_compact(const DevNetRun& net, const uint32_t* __restrict__ rec,
                                            float2* __restrict__ S, const float2* __restrict__ arena,
-                                           uint2* __restrict__ s_head) {
+                                           uint2* __restrict__ s_head, const RecStart& start) {
     const uint32_t tid = threadIdx.x, np = net.n_phases;
-    const uint2* ghead = reinterpret_cast<const uint2*>(rec);
-    const bool staged = np <= kRecHeadSmem;
-    // Phase 0's records follow the headers (rounded up to 16 bytes), so this
-    // thread's first record is loaded together with the headers instead of
-    // after them; the load stays inside the network's records, and the
-    // record is used only if the thread has an element in phase 0.
-    const uint32_t first_word = (2u * np + 3u) & ~3u;
-    const uint4 r0 = first_word + 4u * (tid + 1u) <= net.rec_words
-                         ? __ldg(reinterpret_cast<const uint4*>(rec + first_word) + tid)
-                         : make_uint4(0u, 0u, 0u, 0u);
-    if (staged)
-        for (uint32_t i = tid; i < np; i += blockDim.x) s_head[i] = __ldg(ghead + i);
-    __syncthreads();
-    auto head = [&](uint32_t p) {
-        return p >= np ? make_uint2(0u, 0u) : staged ? s_head[p] : __ldg(ghead + p);
-    };
+    const uint4 r0 = start.first;
+    const RecHeads head = rec_heads(rec, np, start.head, s_head);
     // a phase's header and this thread's record of its first element
     struct Ahead {
         uint2 h;
@@ -744,6 +828,15 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
         if (threadIdx.x == 0) atomicOr(a.status, kStatusQueue);
         return;
     }
+    // the first network's job, where it is known, and the angles (into L1, for
+    // the gate table) travel while the barrier is set up
+    const bool known = !kPersistent || a.static_first;
+    Job job{};
+    if (known && blockIdx.x < a.n_jobs) job = jobs[blockIdx.x];
+    if (kSmemTable && threadIdx.x < a.n_params) {
+        double unused;
+        asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(unused) : "l"(a.params + threadIdx.x));
+    }
     if (threadIdx.x == 0) {
         l2_prefetch_part(a.recs, a.recs_bytes, blockIdx.x, gridDim.x);
         l2_prefetch_part(a.runs, a.runs_bytes, blockIdx.x, gridDim.x);
@@ -776,7 +869,7 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
             if (!table_ready) stage_wait(bar, parity, a.status);   // no copy left in flight
             break;
         }
-        const Job job = jobs[job_i];
+        if (iter > 0 || !known) job = jobs[job_i];
         const DevNetRun& net = job.net;
         // a network with element records needs no blob (shared table and
         // arena only); otherwise blob_capacity 0: the launch reads plan
@@ -789,6 +882,8 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
             if (!table_ready) stage_wait(bar, parity, a.status);
             return;
         }
+        RecStart start{};
+        if (records) start = rec_start(net, a.recs + net.rec_off);
         if (!table_ready) {
             if (!stage_wait(bar, parity, a.status)) return;
             parity ^= 1u;
@@ -805,8 +900,8 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
         float2 term;
         if (!records) term = contract_network<kSmemTable>(net, nblob, table, arena);
         else if (net.rec_format == kRecCompact)
-            term = contract_records_compact(net, a.recs + net.rec_off, stable, arena, s_head);
-        else term = contract_records(net, a.recs + net.rec_off, stable, arena);
+            term = contract_records_compact(net, a.recs + net.rec_off, stable, arena, s_head, start);
+        else term = contract_records(net, a.recs + net.rec_off, stable, arena, s_head, start);
         if (threadIdx.x == 0) {
             *job.term = term;
             if (a.energy) {
@@ -3206,6 +3301,7 @@ int qtb_plan_run(qtb_plan* plan, int32_t first, int32_t count, const double* par
     a.blobs = static_cast<const uint4*>(plan->dev.blobs);
     a.common = static_cast<const uint4*>(plan->dev.entries);
     a.common_bytes = plan->common_bytes;
+    a.n_params = (uint32_t)plan->n_params;
     a.n_entries = (uint32_t)plan->entries.size();
     a.terms_off = plan->common_terms_off;
     a.table_elems = plan->table_elems;
@@ -3526,6 +3622,7 @@ int qtb_plan_run_noalloc(qtb_plan* plan, int32_t first, int32_t count, const dou
     a.blobs = static_cast<const uint4*>(plan->dev.blobs);
     a.common = static_cast<const uint4*>(plan->dev.entries);
     a.common_bytes = plan->common_bytes;
+    a.n_params = (uint32_t)plan->n_params;
     a.n_entries = (uint32_t)n_entries;
     a.terms_off = plan->common_terms_off;
     a.table_elems = plan->table_elems;
