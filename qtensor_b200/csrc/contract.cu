@@ -53,7 +53,7 @@ namespace qtb {
 // (1.8 TB/s of 6.5 for the outer product, 1.2 TB/s for K = 2).  Rows in a
 // block share the load of their b, and with kPairs (N even, 16-byte aligned
 // pointers) two columns load and store 16 bytes.  256 x 256 x 256 outer
-// product: 73.7 -> 24.6 us; K = 2, F = 64, M = N = 512: 116 -> 33 us (134 MB
+// product: 73.7 -> 23.6 us; K = 2, F = 64, M = N = 512: 116 -> 24.9 us (134 MB
 // written; a memset of it takes 20.6 us).
 // I: 32-bit indices, or 64-bit where a dimension needs them.
 template <typename I>
@@ -94,6 +94,14 @@ __device__ __forceinline__ void flat_step(FlatIndex<I>& x, const FlatShape<I>& s
 constexpr int kFlatThreads = 256;
 constexpr int kFlatBlocksPerSm = 4;   // all resident at 64 registers (48 spill: K = 2 41 us; 74 and 8 per SM: 42)
 constexpr int kFlatRows = 4;
+// Outputs from here on are stored evict-first, when pairs of columns are (8-byte
+// stores were not measured and stay plain).  Plain against evict-first, and
+// each with a reduction of the output behind it: K = 2 into 128 MiB 33.1
+// against 24.9 us and 67.9 / 68.1, the outer product 24.8 against 23.7 and
+// 60.0 / 59.8; at 104 MiB 26.8 against 21.0 and 54.6 / 55.2; at 64 MiB, where
+// a reader finds the output in L2, 18.9 against 14.6 but 33.1 / 39.2.
+constexpr uint64_t kFlatStreamBytes = 104ull << 20;
+static bool flat_stream(uint64_t outputs) { return outputs * sizeof(float2) >= kFlatStreamBytes; }
 
 template <typename I>
 static FlatShape<I> flat_shape(uint64_t F, uint64_t M, uint64_t N, int block_rows, int block_cols, unsigned* grid) {
@@ -128,14 +136,23 @@ __device__ __forceinline__ void flat_load(const float2* p, float2 (&v)[kPairs ? 
     }
 }
 
-template <bool kPairs>
+// kStream: evict-first, for an output that L2 (126 MB) does not hold anyway,
+// so that its lines make room for one another as they are written back.
+template <bool kPairs, bool kStream>
 __device__ __forceinline__ void flat_store(float2* p, const float2 (&v)[kPairs ? 2 : 1]) {
-    if constexpr (kPairs) *reinterpret_cast<float4*>(p) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-    else *p = v[0];
+    if constexpr (kPairs) {
+        const float4 q = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        if constexpr (kStream) __stcs(reinterpret_cast<float4*>(p), q);
+        else *reinterpret_cast<float4*>(p) = q;
+    } else if constexpr (kStream) {
+        __stcs(p, v[0]);
+    } else {
+        *p = v[0];
+    }
 }
 
 // c[f,m,n] = a[f,m] * b[f,n].
-template <int kRows, bool kPairs, typename I>
+template <int kRows, bool kPairs, bool kStream, typename I>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_outer_kernel(const float2* __restrict__ a,
                                                                  const float2* __restrict__ b, float2* __restrict__ c,
                                                                  const FlatShape<I> s) {
@@ -156,7 +173,7 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_outer_kern
 #pragma unroll
             for (int e = 0; e < kCols; ++e)
                 p[e] = make_float2(fmaf(u[r].x, v[e].x, -(u[r].y * v[e].y)), fmaf(u[r].y, v[e].x, u[r].x * v[e].y));
-            if (kRows == 1 || m + r < s.M) flat_store<kPairs>(out, p);
+            if (kRows == 1 || m + r < s.M) flat_store<kPairs, kStream>(out, p);
         }
     }
 }
@@ -164,7 +181,7 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_outer_kern
 // C[f,m,n] = sum_k A[k,f,m] B[k,f,n], FP32 sums over k in order.  kAhead k
 // values are loaded together, so that a long sum over few outputs waits for
 // memory once per kAhead terms.
-template <int kRows, bool kPairs, int kAhead, typename I>
+template <int kRows, bool kPairs, bool kStream, int kAhead, typename I>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_contract_simt_kernel(const float2* __restrict__ A,
                                                                          const float2* __restrict__ B,
                                                                          float2* __restrict__ C, uint64_t K,
@@ -213,7 +230,7 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSm) qtb_contract_s
         float2* out = C + (x.f * s.M + m) * s.N + n;
 #pragma unroll
         for (int r = 0; r < kRows; ++r, out += s.N)
-            if (kRows == 1 || m + r < s.M) flat_store<kPairs>(out, sum[r]);
+            if (kRows == 1 || m + r < s.M) flat_store<kPairs, kStream>(out, sum[r]);
     }
 }
 
@@ -678,14 +695,17 @@ int qtb_contract_outer_c64(const void* a, const void* b, void* c, int64_t n, int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int rows = flat_rows((uint64_t)n * m * k, m, k);
     const bool pairs = rows > 1 && k % 2 == 0 && aligned16(b) && aligned16(c);
+    const bool evict = flat_stream((uint64_t)n * m * k);
     unsigned grid = 0;
     if (rows > 1) {
         const FlatShape<uint32_t> s = flat_shape<uint32_t>(n, m, k, rows, pairs ? 2 : 1, &grid);
-        if (pairs) qtb_outer_kernel<kFlatRows, true><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
-        else qtb_outer_kernel<kFlatRows, false><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
+        const auto run = !pairs  ? qtb_outer_kernel<kFlatRows, false, false, uint32_t>
+                        : evict ? qtb_outer_kernel<kFlatRows, true, true, uint32_t>
+                                : qtb_outer_kernel<kFlatRows, true, false, uint32_t>;
+        run<<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
     } else {
         const FlatShape<uint64_t> s = flat_shape<uint64_t>(n, m, k, 1, 1, &grid);
-        qtb_outer_kernel<1, false><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
+        qtb_outer_kernel<1, false, false><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, s);
     }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_outer launch");
@@ -762,17 +782,18 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
         float2* pc = static_cast<float2*>(C);
         const int rows = flat_rows((uint64_t)F * M * N, M, N);
         const bool pairs = rows > 1 && N % 2 == 0 && aligned16(B) && aligned16(C);   // every k's rows too
+        const bool evict = flat_stream((uint64_t)F * M * N);
         const uint64_t as = (uint64_t)F * M, bs = (uint64_t)F * N;
         unsigned grid = 0;
         if (rows > 1) {
             const FlatShape<uint32_t> s = flat_shape<uint32_t>(F, M, N, rows, pairs ? 2 : 1, &grid);
-            if (pairs)
-                qtb_contract_simt_kernel<kFlatRows, true, 2><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
-            else
-                qtb_contract_simt_kernel<kFlatRows, false, 2><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
+            const auto run = !pairs  ? qtb_contract_simt_kernel<kFlatRows, false, false, 2, uint32_t>
+                            : evict ? qtb_contract_simt_kernel<kFlatRows, true, true, 2, uint32_t>
+                                    : qtb_contract_simt_kernel<kFlatRows, true, false, 2, uint32_t>;
+            run<<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
         } else {
             const FlatShape<uint64_t> s = flat_shape<uint64_t>(F, M, N, 1, 1, &grid);
-            qtb_contract_simt_kernel<1, false, 8><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
+            qtb_contract_simt_kernel<1, false, false, 8><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
         }
         e = cudaGetLastError();
         return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");

@@ -60,6 +60,27 @@ def test_simt_sum_edges(cuda_device, K, F, M, N, shift):
     assert np.all(np.abs(got - ref) <= 2 * (K + 4) * EPS * bound + 1e-30)
 
 
+@pytest.mark.parametrize('N', [4096, 4098])
+@pytest.mark.parametrize('K', [1, 3])
+def test_evict_first_line(cuda_device, K, N):
+    # 3 x 1109 rows: just below and just above the size from which outputs
+    # are stored evict-first, with a remainder of rows
+    F, M = 3, 1109
+    assert (F * M * 4096 * 8 < 104 << 20) and (F * M * 4098 * 8 >= 104 << 20)
+    gen = torch.Generator(device=cuda_device).manual_seed(K * N)
+    a = torch.randn((K, F, M), dtype=torch.complex64, device=cuda_device, generator=gen)
+    b = torch.randn((K, F, N), dtype=torch.complex64, device=cuda_device, generator=gen)
+    c = torch.full((F, M, N), complex(np.nan, 0), dtype=torch.complex64, device=cuda_device)
+    if K == 1:
+        tcontract.mkl_contract_complex(a[0], b[0], c)
+    else:
+        tcontract.mkl_contract_sum(a, b, c, mode='simt')
+    for f in range(F):
+        ref = a[:, f].to(torch.complex128).T @ b[:, f].to(torch.complex128)
+        bound = a[:, f].abs().double().T @ b[:, f].abs().double()
+        assert bool(((c[f] - ref).abs() <= 2 * (K + 4) * EPS * bound).all())
+
+
 @pytest.mark.parametrize('u,sum_first', [(17, 1), (17, 0), (18, 1), (19, 0), (21, 1)])
 @pytest.mark.parametrize('shift', [0, 1])
 def test_large_bucket_edges(cuda_device, u, sum_first, shift):
