@@ -337,7 +337,7 @@ int qtb_plan_set_dynamic_claims(qtb_plan* plan, int32_t enable);
 /* Launch classes of the plan's most recent run: 4 ints per class (networks,
  * threads per CTA, dynamic shared memory bytes, flags: 1 = shared-memory
  * arena, 2 = persistent launch taking networks from a queue, 4 = a wave of
- * wide networks contracted by the whole GPU step by step, arenas in
+ * wide networks, a team of CTAs contracting each phase by phase, arenas in
  * scratch, 8 = lean persistent queue (registers capped), 16 = warp-per-
  * network queue, 32 = the 96-thread lean queue, 64 = networks of moderate
  * size, one thread-block cluster each, arenas in scratch, 128 = networks

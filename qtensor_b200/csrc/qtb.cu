@@ -16,9 +16,9 @@
 //                            with the MaxCut post-processing
 //                            (QAOASimulator.py:27-41); class, persistent,
 //                            lean-persistent and hybrid schedules
-//   K4  qtb_wide_kernel      networks too large for shared memory, in waves
-//                            contracted by the whole GPU one elimination
-//                            phase at a time (tile queue, bounded waits)
+//   K4  qtb_wide_kernel      networks too large for shared memory, in waves:
+//                            a team of CTAs per network takes the tiles of
+//                            its phases in order (bounded waits)
 //   K0  qtb_table_kernel     the gate table in global memory, for plans whose
 //                            table does not fit in shared memory and for
 //                            wide waves
@@ -1808,12 +1808,12 @@ static void launch_bucket(const BucketArgs& a, cudaStream_t st) {
 // separated by the cluster barrier (release/acquire at cluster scope, after
 // a fence for the arena in global memory).  A cluster's CTAs are scheduled
 // together by the hardware, so the barrier needs no flag and no co-residency
-// assumption, unlike the grid-wide steps of K4; a network's critical path
+// assumption, unlike the teams of K4; a network's critical path
 // is its phase chain at cluster-barrier latency, and the networks of a run
 // proceed independently.  The arena lives in global memory (read with
 // ld.cg: another CTA wrote it), the plan blob is read through the read-only
 // path.  A chunk that lies within one op of at least 2048 elements is
-// computed with the batched loads of K4 (eight elements per thread).
+// computed with batched loads (eight elements per thread).
 struct ClusterJob {
     const DevNetRun* run;
     float2* term;

@@ -193,8 +193,8 @@ class QAOAEnergyEngine:
     records: resolve every output element's operand offsets on the host, so
     that the shared-memory executor only loads and multiplies (same
     products, same order; off: the executor decodes the plan blobs).
-    wave_ctas_per_sm: resident CTAs per SM of the wide networks' whole-GPU
-    waves (0: as many as fit).
+    wave_ctas_per_sm: halves of every SM that the wide networks' waves may
+    hold (0: both).
     dynamic_claims: persistent launches claim every network from their
     queue (for a GPU shared with other streams' kernels; off: each CTA starts
     on the job of its own index, which saves a queue round trip when the

@@ -187,7 +187,7 @@ class NetworkPlan:
                                            nbytes, ctypes.c_void_p(int(stream))))
 
     def set_wave_ctas_per_sm(self, ctas):
-        """Resident CTAs per SM of the wide waves (0: as many as fit); set
+        """Halves of every SM that the wide waves may hold (0: both); set
         before the first run."""
         check(self._lib.qtb_plan_set_wave_ctas_per_sm(self._h, int(ctas)))
 

@@ -120,8 +120,8 @@ class QAOAServer:
     candidates they bring), fewer than the engine's 16 because a request's
     compile is on its latency path.  compile_workers: host threads compiling
     requests concurrently, each with compile_threads C++ threads (default:
-    its share of the CPUs the process may use).  wave_ctas_per_sm: resident
-    CTAs per SM of a wide request's whole-GPU waves (1 leaves half of every
+    its share of the CPUs the process may use).  wave_ctas_per_sm: halves
+    of every SM that a wide request's waves may hold (1 leaves half of every
     SM to the other requests' kernels while a wide request runs; 0 lets
     the waves take whole SMs).  Every request's persistent launches claim
     all their networks from their queues (the engine's dynamic_claims): with
