@@ -3439,7 +3439,8 @@ int qtb_plan_run_plain(qtb_plan* plan, int32_t first, int32_t count, const doubl
             a.k = op.k;
             a.sum = op.sum;
             a.w = op.u - op.sum;
-            launch_bucket(a, st);
+            // never by the chunks of K4, which this path is the check of
+            qtb_bucket_kernel<<<bucket_blocks(a.w), kBucketThreads, 0, st>>>(a);
             QTB_CUDA(cudaGetLastError());
         }
         const float2* res = (net.result_src & kSrcTable) ? table + (net.result_src & ~kSrcTable)
