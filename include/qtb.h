@@ -364,6 +364,13 @@ int qtb_plan_device_status(qtb_plan* plan, int32_t* status);
  * spin_limit polls it gives up and sets QTB_STATUS_WAIT_TIMEOUT in a status
  * word returned in *status_out.  Synchronous; the device stays usable.    */
 int qtb_selftest_wait_timeout(int32_t spin_limit, int32_t* status_out);
+/* The same for the tensor-core contract-sum (arguments as in
+ * qtb_contract_sum_c64 with mode 2): the CTAs of part `part` of a K that is
+ * split (0 .. parts - 1, else an error) stage nothing, so that their waits
+ * run out after spin_limit polls.  The status word becomes 2, and no output
+ * of those CTAs' tiles is written.  Asynchronous on stream.              */
+int qtb_selftest_contract_timeout(const void* A, const void* B, void* C, int64_t K, int64_t F, int64_t M, int64_t N,
+                                  void* scratch, size_t scratch_bytes, int32_t spin_limit, int32_t part, void* stream);
 
 /* Device pointer of pinned host memory (cudaHostGetDevicePointer), so that
  * kernels read a caller's pinned angles and write its pinned energy

@@ -370,10 +370,10 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, 
         "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
-// Bounded wait for the mbarrier phase `parity`; false after the limit.
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
+// Bounded wait for the mbarrier phase `parity`; false after `limit` polls.
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
     uint32_t done = 0;
-    for (uint32_t it = 0; it < kTcSpinLimit; ++it) {
+    for (uint32_t it = 0; it < limit; ++it) {
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
             " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
@@ -439,7 +439,9 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 // epilogue thread).  Every wait is bounded; on a timeout the status word is
 // set, every role stops, and the CTA waits (bounded, in phase order) for its
 // copies and MMAs in flight before freeing TMEM; it still meets its
-// cluster's barriers.
+// cluster's barriers, and no CTA of the cluster stores its part of the tile,
+// whose sums are not finished.  kTest: the self-test's, whose CTAs of rank
+// `stall` stage nothing and whose waits run out after spin_limit polls.
 // What bounds it: shared memory.  A 128 x 128 tile's six MMAs take 768 tensor
 // cycles per 8 k, read 72 KB of operands and see 40 KB written: 875 cycles at
 // 128 bytes each (measured about 1100).  128 x 64 tiles with B stored as both
@@ -448,11 +450,12 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 // (4 CTAs per tile in place of 27 serial ones).  Measured and not kept: B as
 // [Br | Bi] with the negative products through the descriptor's negate-A bit
 // (32 KB per tile but N = 128 MMAs, 128 operand bytes per cycle: 116 us).
-template <uint32_t kN>
+template <uint32_t kN, bool kTest>
 __global__ void __launch_bounds__(TcTile<kN>::kThreads, 1)
 qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restrict__ Bp, float2* __restrict__ C,
                        uint32_t M, uint32_t N, uint32_t row_tiles, uint32_t col_tiles, uint32_t k_blocks,
-                       uint32_t split, uint32_t vec, int* status) {
+                       uint32_t split, uint32_t vec, int* status, uint32_t spin_limit, uint32_t stall) {
+    const uint32_t limit = kTest ? spin_limit : kTcSpinLimit;
     using T = TcTile<kN>;
     constexpr uint32_t NS = T::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -501,9 +504,9 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
             const uint32_t* a_f = Ap + (((uint64_t)f * row_tiles + mt) * k_tiles + kt0) * (kTcAPlanes * kTcAWords);
             const uint32_t* b_f = Bp + (((uint64_t)f * col_tiles + nt) * k_tiles + kt0) * (kTcBPlanes * T::kBWords);
             uint32_t loaded = 0;
-            for (; loaded < n_tiles && s_ok; ++loaded) {   // tile `loaded` into stage loaded % NS
+            for (; loaded < n_tiles && s_ok && !(kTest && rank == stall); ++loaded) {   // tile `loaded` into stage loaded % NS
                 const uint32_t s = loaded % NS;
-                if (loaded >= NS && !tc_wait(empty(s), (loaded / NS - 1u) & 1u)) {
+                if (loaded >= NS && !tc_wait(empty(s), (loaded / NS - 1u) & 1u, limit)) {
                     fail_once();   // the MMAs have not read the stage's previous tile
                     break;
                 }
@@ -518,7 +521,8 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
             }
             // no copy may still write shared memory when it is reused: wait
             // (bounded) for each stage's last one
-            for (uint32_t i = loaded > NS ? loaded - NS : 0u; i < loaded; ++i) tc_wait(full(i % NS), (i / NS) & 1u);
+            for (uint32_t i = loaded > NS ? loaded - NS : 0u; i < loaded; ++i)
+                tc_wait(full(i % NS), (i / NS) & 1u, kTcSpinLimit);
         }
         __syncwarp();
     } else if (warp == T::kEpilogueWarps) {   // the MMAs
@@ -527,11 +531,11 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
             for (uint32_t i = 0; i < n_tiles && s_ok; ++i) {
                 const uint32_t s = i % NS, b = i / kTcStagesPerBlock, buf = b & 1u;
                 const bool block_first = i % kTcStagesPerBlock == 0;
-                if (block_first && b >= 2 && !tc_wait(tempty(buf), ((b - 2) >> 1) & 1u)) {
+                if (block_first && b >= 2 && !tc_wait(tempty(buf), ((b - 2) >> 1) & 1u, limit)) {
                     fail_once();   // the epilogue has not read this buffer's previous block
                     break;
                 }
-                if (!tc_wait(full(s), (i / NS) & 1u)) {
+                if (!tc_wait(full(s), (i / NS) & 1u, limit)) {
                     fail_once();
                     break;
                 }
@@ -557,7 +561,7 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
             // no MMA may still read shared memory or write TMEM when they are
             // reused or freed: wait (bounded) for each stage's last commit
             for (uint32_t i = committed > NS ? committed - NS : 0u; i < committed; ++i)
-                tc_wait(empty(i % NS), (i / NS) & 1u);
+                tc_wait(empty(i % NS), (i / NS) & 1u, kTcSpinLimit);
         }
         __syncwarp();
     } else {
@@ -568,7 +572,7 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
         for (uint32_t b = 0; b < n_blocks; ++b) {
             const uint32_t buf = b & 1u;
             if (!s_ok) break;
-            if (!tc_wait(tfull(buf), (b >> 1) & 1u)) {
+            if (!tc_wait(tfull(buf), (b >> 1) & 1u, limit)) {
                 fail_once();
                 break;
             }
@@ -602,7 +606,13 @@ qtb_tc_contract_kernel(const uint32_t* __restrict__ Ap, const uint32_t* __restri
     cluster_sync();
     // rows rank, rank + split, ... of the tile, the CTAs' sums added in rank
     // order; a warp stores whole rows, two columns per lane
-    const uint32_t ok = s_ok;
+    uint32_t ok = s_ok;
+    for (uint32_t q = 0; q < split && split > 1; ++q) {   // a CTA that gave up leaves its part of the sums out
+        uint32_t peer, peer_ok;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(tc_smem(const_cast<const int*>(&s_ok))), "r"(q));
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(peer_ok) : "r"(peer) : "memory");
+        ok &= peer_ok;
+    }
     for (uint32_t r = rank + warp * split; r < kTcM; r += (T::kEpilogueWarps + 2) * split) {
         const uint32_t m = mt * kTcM + r;
         if (m >= M) break;
@@ -726,9 +736,9 @@ int qtb_contract_sum_scratch_bytes(int64_t K, int64_t F, int64_t M, int64_t N, i
 
 }  // extern "C"
 
-template <uint32_t kN>
+template <uint32_t kN, bool kTest>
 static cudaError_t tc_launch(const TcShape& t, const float2* A, const float2* B, float2* C, int64_t K, int64_t F,
-                             int64_t M, int64_t N, void* scratch, cudaStream_t st) {
+                             int64_t M, int64_t N, void* scratch, cudaStream_t st, uint32_t spin_limit, uint32_t stall) {
     using T = TcTile<kN>;
     int* status = static_cast<int*>(scratch);
     const uint64_t k_tiles = t.k_blocks * kTcStagesPerBlock;
@@ -740,7 +750,7 @@ static cudaError_t tc_launch(const TcShape& t, const float2* A, const float2* B,
         A, B, reinterpret_cast<uint4*>(Ap), reinterpret_cast<uint4*>(Bp), (uint32_t)K, (uint32_t)F, (uint32_t)M,
         (uint32_t)N, (uint32_t)k_tiles, (uint32_t)t.row_tiles, (uint32_t)t.col_tiles, (uint32_t)a_blocks, status);
     // per device and cheap: set on every call
-    cudaError_t e = cudaFuncSetAttribute(qtb_tc_contract_kernel<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(qtb_tc_contract_kernel<kN, kTest>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)T::kSmemBytes);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
@@ -758,9 +768,25 @@ static cudaError_t tc_launch(const TcShape& t, const float2* A, const float2* B,
     cfg.attrs = attr;
     cfg.numAttrs = t.split > 1 ? 2 : 1;
     const uint32_t vec = N % 2 == 0 && aligned16(C);
-    return cudaLaunchKernelEx(&cfg, qtb_tc_contract_kernel<kN>, (const uint32_t*)Ap, (const uint32_t*)Bp, C, (uint32_t)M,
+    return cudaLaunchKernelEx(&cfg, qtb_tc_contract_kernel<kN, kTest>, (const uint32_t*)Ap, (const uint32_t*)Bp, C, (uint32_t)M,
                               (uint32_t)N, (uint32_t)t.row_tiles, (uint32_t)t.col_tiles, (uint32_t)t.k_blocks, t.split,
-                              vec, status);
+                              vec, status, spin_limit, stall);
+}
+
+// The tensor-core contract-sum; arguments and scratch size checked by the caller.
+template <bool kTest>
+static int tc_sum(const TcShape& t, const void* A, const void* B, void* C, int64_t K, int64_t F, int64_t M, int64_t N,
+                  void* scratch, cudaStream_t st, uint32_t spin_limit = 0, uint32_t stall = 0) {
+    const uint64_t k_tiles = t.k_blocks * kTcStagesPerBlock;
+    if (t.row_tiles > 65535 || F > 65535 || t.col_tiles * t.split > (1u << 30) || K > (1ll << 30) ||
+        (uint64_t)F * (t.row_tiles + t.col_tiles) * k_tiles >= (1ull << 31))
+        return fail(QTB_ERR_UNSUPPORTED, "contract_sum: shape beyond the tensor-core grid");
+    const float2 *pa = static_cast<const float2*>(A), *pb = static_cast<const float2*>(B);
+    float2* pc = static_cast<float2*>(C);
+    cudaError_t e = t.n == 128 ? tc_launch<128, kTest>(t, pa, pb, pc, K, F, M, N, scratch, st, spin_limit, stall)
+                               : tc_launch<64, kTest>(t, pa, pb, pc, K, F, M, N, scratch, st, spin_limit, stall);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
 }
 
 extern "C" {
@@ -776,7 +802,6 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
     if (!scratch || scratch_bytes < need)
         return fail(QTB_ERR_ARG, "contract_sum: scratch smaller than qtb_contract_sum_scratch_bytes");
     int* status = static_cast<int*>(scratch);
-    cudaError_t e = cudaSuccess;
     if (!use_tensor_cores(mode, K, M, N)) {
         const float2 *pa = static_cast<const float2*>(A), *pb = static_cast<const float2*>(B);
         float2* pc = static_cast<float2*>(C);
@@ -795,20 +820,26 @@ int qtb_contract_sum_c64(const void* A, const void* B, void* C, int64_t K, int64
             const FlatShape<uint64_t> s = flat_shape<uint64_t>(F, M, N, 1, 1, &grid);
             qtb_contract_simt_kernel<1, false, false, 8><<<grid, kFlatThreads, 0, st>>>(pa, pb, pc, K, as, bs, status, s);
         }
-        e = cudaGetLastError();
+        const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
     }
+    return tc_sum<false>(tc_shape(K, F, M, N), A, B, C, K, F, M, N, scratch, st);
+}
+
+int qtb_selftest_contract_timeout(const void* A, const void* B, void* C, int64_t K, int64_t F, int64_t M, int64_t N,
+                                  void* scratch, size_t scratch_bytes, int32_t spin_limit, int32_t part, void* stream) {
+    if (!A || !B || !C || K < 1 || F < 1 || M < 1 || N < 1 || spin_limit < 1 || part < 0)
+        return fail(QTB_ERR_ARG, "selftest_contract_timeout: bad arguments");
+    size_t need = 0;
+    int r = qtb_contract_sum_scratch_bytes(K, F, M, N, 2, &need);
+    if (r) return r;
+    if (!scratch || scratch_bytes < need)
+        return fail(QTB_ERR_ARG, "selftest_contract_timeout: scratch smaller than qtb_contract_sum_scratch_bytes");
     const TcShape t = tc_shape(K, F, M, N);
-    const uint64_t k_tiles = t.k_blocks * kTcStagesPerBlock;
-    if (t.row_tiles > 65535 || F > 65535 || t.col_tiles * t.split > (1u << 30) || K > (1ll << 30) ||
-        (uint64_t)F * (t.row_tiles + t.col_tiles) * k_tiles >= (1ull << 31))
-        return fail(QTB_ERR_UNSUPPORTED, "contract_sum: shape beyond the tensor-core grid");
-    const float2 *pa = static_cast<const float2*>(A), *pb = static_cast<const float2*>(B);
-    float2* pc = static_cast<float2*>(C);
-    e = t.n == 128 ? tc_launch<128>(t, pa, pb, pc, K, F, M, N, scratch, st)
-                   : tc_launch<64>(t, pa, pb, pc, K, F, M, N, scratch, st);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    return e == cudaSuccess ? QTB_OK : cuda_fail_c(e, "contract_sum launch");
+    if ((uint32_t)part >= t.split)
+        return fail(QTB_ERR_ARG, "selftest_contract_timeout: the shape's K is in " + std::to_string(t.split) + " parts");
+    return tc_sum<true>(t, A, B, C, K, F, M, N, scratch, static_cast<cudaStream_t>(stream), (uint32_t)spin_limit,
+                        (uint32_t)part);
 }
 
 }  // extern "C"

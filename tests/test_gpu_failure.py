@@ -34,3 +34,37 @@ def test_selftest_rejects_bad_arguments(cuda_device):
     status = ctypes.c_int32(0)
     assert _lib.lib().qtb_selftest_wait_timeout(0, ctypes.byref(status)) == _lib.QTB_ERR_ARG
     assert _lib.lib().qtb_selftest_wait_timeout(16, None) == _lib.QTB_ERR_ARG
+
+
+@pytest.mark.parametrize('K,F,M,N,parts', [(544, 1, 100, 60, 8), (894, 4, 1309, 574, 2)])
+def test_contract_timeout_leaves_the_tile_unwritten(cuda_device, K, F, M, N, parts):
+    """K of one tile is split over `parts` CTAs; where one of them gives up,
+    its part is missing from the tile's sums, so the others store nothing
+    either (every row of the output keeps what it held)."""
+    import numpy as np
+    import torch
+    from qtensor_b200 import _lib, tcontract
+    lib = _lib.lib()
+    gen = torch.Generator(device=cuda_device).manual_seed(K)
+    a = torch.randn((K, F, M), dtype=torch.complex64, device=cuda_device, generator=gen)
+    b = torch.randn((K, F, N), dtype=torch.complex64, device=cuda_device, generator=gen)
+    c = torch.full((F, M, N), complex(np.nan, 0), dtype=torch.complex64, device=cuda_device)
+    scratch = torch.empty(tcontract.contract_sum_scratch_bytes(K, F, M, N, 'tensor'), dtype=torch.uint8,
+                          device=cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(part):
+        return lib.qtb_selftest_contract_timeout(a.data_ptr(), b.data_ptr(), c.data_ptr(), K, F, M, N,
+                                                 scratch.data_ptr(), scratch.numel(), 1 << 14, part, stream)
+
+    assert run(parts) == _lib.QTB_ERR_ARG
+    for part in (0, parts - 1):
+        _lib.check(run(part))
+        torch.cuda.synchronize()
+        assert int(scratch[:4].view(torch.int32).item()) == 2
+        assert bool(torch.isnan(c.real).all())
+    # the device and the scratch are as good as before
+    tcontract.mkl_contract_sum(a, b, c, mode='tensor', scratch=scratch)
+    ref = a.to(torch.complex128).permute(1, 2, 0) @ b.to(torch.complex128).permute(1, 0, 2)
+    assert int(scratch[:4].view(torch.int32).item()) == 0
+    assert (c - ref).abs().max().item() <= 1e-5 * ref.abs().max().item()
