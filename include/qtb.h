@@ -314,9 +314,9 @@ int qtb_plan_run_plain(qtb_plan* plan, int32_t first, int32_t count, const doubl
  * memory, classes concurrent) with 64..1024 threads per CTA, then the whole
  * class schedule against the persistent, hybrid (large networks as
  * classes + a lean persistent queue) and warp-per-network schedules, and
- * keeps the fastest; later runs reuse the choices.  A range with wide
- * networks keeps the class schedule and its default block sizes: their
- * waves outlast the other networks' launches.
+ * keeps the fastest; later runs reuse the choices.  A range whose work lies
+ * mostly in wide networks is not timed: it keeps the class schedule and its
+ * default block sizes.
  * QTB_AUTOTUNE=0 in the environment keeps the default block sizes;
  * QTB_SCHEDULE fixes the schedule.                                       */
 int qtb_plan_set_autotune(qtb_plan* plan, int32_t enable);

@@ -1969,6 +1969,8 @@ struct RunCache {
     std::vector<WideWave> waves;        // wide networks (both schedules), run one after another
     void* wide_buf = nullptr;
     size_t zeroed_off = 0, zeroed_bytes = 0;   // counters of all waves, zeroed before a run
+    double wave_us = 0.0, wave_flops = 0.0;    // the waves' modelled time, their networks' work
+    double smem_flops = 0.0;                   // work of the networks in shared memory
     size_t scratch_elems = 0;           // arenas of the largest wave, then the cluster arenas
     void* cl_jobs = nullptr;            // ClusterJob per network of moderate size (K5)
     int n_cl = 0;
@@ -2271,6 +2273,7 @@ constexpr size_t kWideWaveBytes = size_t(1) << 30;
 // The tables of one wave's networks `members` (see WideNet ...); `slots`:
 // resident CTAs, which are shared out in teams.
 struct WideTables {
+    double us = 0.0;   // modelled time
     std::vector<WideStep> steps;
     std::vector<WideItem> items;
     std::vector<uint32_t> tile_item, tickets;
@@ -2303,8 +2306,9 @@ static WideCut wide_cut(uint64_t chunks, uint64_t small, uint64_t team) {
 // team), (0.6 + 0.4 k) us per chunk of an op of k operands, 2.5 us per 256
 // elements of small ops, 0.8 us per phase of a chain (3 or 5.5 us per tile in
 // its place: 379 and 509 us on the two graphs at qtb_wide_kernel, 8 us 382 and
-// 492 us).
-static std::vector<uint32_t> wide_teams(const qtb_plan* plan, const std::vector<int32_t>& members, uint64_t slots) {
+// 492 us).  *us: that time.
+static std::vector<uint32_t> wide_teams(const qtb_plan* plan, const std::vector<int32_t>& members, uint64_t slots,
+                                        double* us) {
     constexpr double kTileUs = 8.0, kSmallUs = 2.5, kChainUs = 0.8;
     struct Load {
         uint64_t chunks, small;
@@ -2384,13 +2388,14 @@ static std::vector<uint32_t> wide_teams(const qtb_plan* plan, const std::vector<
             lo = mid;
         }
     }
+    *us = hi;
     return teams;
 }
 
 static WideTables wave_tables(const qtb_plan* plan, const std::vector<int32_t>& members, uint64_t slots,
                               std::vector<WideNet>* nets) {
-    const std::vector<uint32_t> teams = wide_teams(plan, members, slots);
     WideTables out;
+    const std::vector<uint32_t> teams = wide_teams(plan, members, slots, &out.us);
     for (size_t k = 0; k < members.size(); ++k) {
         const Network& n = plan->nets[members[k]];
         const DevNetRun& run = plan->druns[members[k]];
@@ -2481,6 +2486,7 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
                        RunCache* rc, bool device) {
     rc->waves.clear();
     rc->zeroed_bytes = 0;
+    rc->wave_us = rc->wave_flops = 0.0;
     if (wide.empty()) return QTB_OK;
     auto arena_of = [&](int32_t i) { return ((size_t)plan->druns[i].arena_elems + 63) & ~size_t(63); };
     std::stable_sort(wide.begin(), wide.end(), [&](int32_t x, int32_t y) { return arena_of(x) > arena_of(y); });
@@ -2521,6 +2527,8 @@ static int build_waves(qtb_plan* plan, std::vector<int32_t> wide, int32_t first,
                 off += arena_of(members[k]);
             }
             WideTables tb = wave_tables(plan, members, slots, &wn);
+            rc->wave_us += tb.us;
+            for (int32_t i : members) rc->wave_flops += plan->nets[i].info.alg_flops;
             WideWave wv{};
             wv.n_nets = (uint32_t)members.size();
             wv.n_tickets = (uint32_t)tb.tickets.size();
@@ -2656,6 +2664,8 @@ static int build_run(qtb_plan* plan, int32_t first, int32_t count, float2* terms
     // (largest arena, then most phases) first
     std::vector<int32_t> all;
     for (int c = 0; c < kSmemClasses; ++c) all.insert(all.end(), members[c].begin(), members[c].end());
+    rc->smem_flops = 0.0;
+    for (int32_t i : all) rc->smem_flops += plan->nets[i].info.alg_flops;
     std::stable_sort(all.begin(), all.end(), [&](int32_t x, int32_t y) {
         const DevNetRun& rx = plan->druns[x];
         const DevNetRun& ry = plan->druns[y];
@@ -3023,19 +3033,37 @@ static int launch_schedule(qtb_plan_device* s, const RunCache* rc,
     return QTB_OK;
 }
 
+// Whether the launches beside a range's waves are worth timing: the work
+// outside the waves has to be the larger part and, at about 3 MFLOP per us, to
+// take a sixth of the waves' modelled time.  Default classes against the best
+// other schedule, measured as whole calls: one wide network (modelled 151 us)
+// beside 1500 small ones (93 MFLOP) 133 / 117-124 us, beside 4500 167 / 118,
+// beside 9000 224 / 146; beside 239 (29 MFLOP) 123 / 115-118, beside 89 (13
+// MFLOP) 107.7 / 106.9.  What the autotuner then picks: 115-134, 160, 150-207
+// us (it times launches, whose host part a captured call does not have).
+// Where the waves are the larger part no schedule is reliably better and the
+// timing misleads (classes / hybrid, two runs each): N=256 p=4 375 / 373-396
+// us, N=300 p=4 341 / 327-368, Erdos-Renyi N=400 p=3 503 / 509-513, N=300 322 /
+// 294.  The timing takes 18-30 ms of a first run.
+static bool tune_beside_waves(const RunCache* rc) {
+    return rc->smem_flops >= rc->wave_flops && rc->smem_flops / 3e6 >= rc->wave_us / 6.0;
+}
+
 // Autotuner, on the first run of a range (energy reduction off while it
 // times): each class of the class schedule is timed alone with 64..1024
 // threads per CTA; then the whole class schedule and the persistent
 // schedule (128/256/512 threads) are timed end to end and the faster
 // schedule is kept.  Each measurement is the fastest of three launches.
+// Beside waves the class schedule is timed with its default blocks too: a
+// block that is best for a class alone need not be beside a wave.
 static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, void* scratch_dev,
                         cudaStream_t st) {
     static const int kCandidates[] = {64, 128, 256, 512, 1024};
-    if (!rc->waves.empty()) {
-        // a wave outlasts the other networks' launches, which run in its
-        // shadow; timed beside it they differ by less than the launch order
-        // does (a tuned choice took between 456 and 645 us on N=256 p=4,
-        // the classes with their default blocks 432 us on every run)
+    const bool log = std::getenv("QTB_AUTOTUNE_LOG") != nullptr;
+    if (!rc->waves.empty() && !tune_beside_waves(rc)) {
+        if (log)
+            std::fprintf(stderr, "qtb autotune: waves (%.0f us by the model, %.1f MFLOP) beside %.1f MFLOP -> classes, "
+                         "not timed\n", rc->wave_us, 1e-6 * rc->wave_flops, 1e-6 * rc->smem_flops);
         rc->schedule = kSchedClasses;
         rc->tuned = true;
         return QTB_OK;
@@ -3045,7 +3073,6 @@ static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, v
     QTB_CUDA(cudaEventCreate(&e1));
     RunArgs a = base;
     a.energy = nullptr;
-    const bool log = std::getenv("QTB_AUTOTUNE_LOG") != nullptr;
     auto time_it = [&](auto&& launch, float* best) -> int {
         int r = launch();   // warm-up
         if (r) return r;
@@ -3061,6 +3088,11 @@ static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, v
         return QTB_OK;
     };
     int r;
+    const std::vector<LaunchClass> default_classes = rc->classes;
+    float default_ms = 1e30f;
+    if (!rc->waves.empty() &&
+        (r = time_it([&] { return launch_schedule(s, rc, default_classes, a, scratch_dev, st); }, &default_ms)))
+        return r;
     for (LaunchClass& lc : rc->classes) {
         int best_t = lc.threads;
         float best_ms = 1e30f;
@@ -3085,6 +3117,10 @@ static int autotune_run(qtb_plan_device* s, RunCache* rc, const RunArgs& base, v
     float class_ms = 1e30f;
     if ((r = time_it([&] { return launch_schedule(s, rc, rc->classes, a, scratch_dev, st); }, &class_ms)))
         return r;
+    if (default_ms < class_ms) {
+        rc->classes = default_classes;
+        class_ms = default_ms;
+    }
     float pers_ms = 1e30f;
     if (!rc->pclasses.empty()) {
         for (LaunchClass& pc : rc->pclasses) {
