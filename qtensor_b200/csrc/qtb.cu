@@ -352,26 +352,41 @@ __device__ __forceinline__ void neumaier_add(double& sum, double& comp, double x
 // fence that the end of the kernel makes needless); so 3.6 us and 1.4 us.
 constexpr uint32_t kSumLanes = 128, kSumGroups = kSumLanes / 32;
 
-// (sum, compensation) of group g of 32 running sums, in every lane of a warp.
-__device__ __forceinline__ double2 reduce_group(const float2* terms, uint32_t n, uint32_t g) {
-    constexpr uint32_t kBatch = 12;   // loads in flight per lane
-    double s = 0.0, c = 0.0;
-    for (uint32_t base = g * 32u + (threadIdx.x & 31u); base < n; base += kSumLanes * kBatch) {
-        float x[kBatch];
+// (sum, compensation) of kG groups of 32 running sums from group g0 on, in
+// every lane of a warp.  The groups of a warp advance together, since a chain
+// of dependent fp64 additions is what a group costs: one warp that took its
+// four groups in turn made warp:64 schedules 116 -> 123 us per call on N=1000
+// p=3.  A compensation is far smaller than its sum, so that compensations are
+// added without one of their own.
+template <uint32_t kG>
+__device__ __forceinline__ void reduce_groups(const float2* terms, uint32_t n, uint32_t g0, double2 (&group)[kG]) {
+    constexpr uint32_t kBatch = kG == 1 ? 12 : 4;   // loads of a group in flight per lane
+    double s[kG] = {}, c[kG] = {};
+    for (uint32_t base = g0 * 32u + (threadIdx.x & 31u); base < n; base += kSumLanes * kBatch) {
+        float x[kBatch][kG];
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j)
-            x[j] = base + kSumLanes * j < n ? __ldcg(&terms[base + kSumLanes * j].x) : 0.f;
+#pragma unroll
+            for (uint32_t g = 0; g < kG; ++g) {
+                const uint32_t i = base + kSumLanes * j + 32u * g;
+                x[j][g] = i < n ? __ldcg(&terms[i].x) : 0.f;
+            }
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j)
-            if (base + kSumLanes * j < n) neumaier_add(s, c, (double)x[j]);
+#pragma unroll
+            for (uint32_t g = 0; g < kG; ++g)
+                if (base + kSumLanes * j + 32u * g < n) neumaier_add(s[g], c[g], (double)x[j][g]);
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        const double os = __shfl_xor_sync(0xffffffffu, s, off);
-        const double oc = __shfl_xor_sync(0xffffffffu, c, off);
-        neumaier_add(s, c, os);
-        c += oc;
-    }
-    return make_double2(s, c);
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (uint32_t g = 0; g < kG; ++g) {
+            const double os = __shfl_xor_sync(0xffffffffu, s[g], off);
+            const double oc = __shfl_xor_sync(0xffffffffu, c[g], off);
+            neumaier_add(s[g], c[g], os);
+            c[g] += oc;
+        }
+#pragma unroll
+    for (uint32_t g = 0; g < kG; ++g) group[g] = make_double2(s[g], c[g]);
 }
 
 __device__ __forceinline__ void reduce_finish(const double2 (&group)[kSumGroups], double n_groups, double* energy) {
@@ -387,10 +402,9 @@ __device__ __forceinline__ void reduce_finish(const double2 (&group)[kSumGroups]
 }
 
 // By one warp (all 32 lanes call it).
-__device__ void reduce_energy_warp(const float2* terms, uint32_t n, double n_groups, double* energy) {
+__device__ __noinline__ void reduce_energy_warp(const float2* terms, uint32_t n, double n_groups, double* energy) {
     double2 group[kSumGroups];
-#pragma unroll
-    for (uint32_t g = 0; g < kSumGroups; ++g) group[g] = reduce_group(terms, n, g);
+    reduce_groups(terms, n, 0u, group);
     if ((threadIdx.x & 31u) == 0) reduce_finish(group, n_groups, energy);
 }
 
@@ -400,8 +414,9 @@ __device__ void reduce_energy(const float2* terms, uint32_t n, double n_groups, 
     __shared__ double2 s_group[kSumGroups];
     const uint32_t warps = blockDim.x >> 5;
     for (uint32_t g = threadIdx.x >> 5; g < kSumGroups; g += warps) {
-        const double2 v = reduce_group(terms, n, g);
-        if ((threadIdx.x & 31u) == 0) s_group[g] = v;
+        double2 v[1];
+        reduce_groups(terms, n, g, v);
+        if ((threadIdx.x & 31u) == 0) s_group[g] = v[0];
     }
     __syncthreads();
     if (threadIdx.x == 0) {
