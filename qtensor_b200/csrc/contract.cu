@@ -144,9 +144,8 @@ __device__ __forceinline__ void flat_store(float2* p, const float2 (&v)[kPairs ?
         const float4 q = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
         if constexpr (kStream) __stcs(reinterpret_cast<float4*>(p), q);
         else *reinterpret_cast<float4*>(p) = q;
-    } else if constexpr (kStream) {
-        __stcs(p, v[0]);
     } else {
+        static_assert(!kStream, "single columns are stored plainly");
         *p = v[0];
     }
 }
