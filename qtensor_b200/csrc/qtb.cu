@@ -824,9 +824,18 @@ __device__ float2 contract_records_compact(const DevNetRun& net, const uint32_t*
 //   so small networks keep twice as many in flight per SM; kLean 2 (96
 //   threads, 12 CTAs per SM) for networks whose staging and arena fit a
 //   twelfth of an SM, so that a run of N=1000 p=3 size is resident at once.
-template <bool kSmemArena, bool kSmemTable, bool kPersistent, int kLean = 0>
+//   kForm, of persistent launches with arena and table in shared memory: the
+//   wide records' loads two phases ahead take kFormAny to 96 registers, 5 CTAs
+//   of 128 threads per SM where 8 fit before, and the 96-thread queue to 44
+//   bytes of spills.  kFormCompact, for queues whose every network has compact
+//   records, is the body without the other formats (61 registers; no spills at
+//   the 56 of the 96-thread queue), kFormCapped all formats in 64 registers
+//   (the records' words move about); see persistent_grid.
+constexpr int kFormAny = 0, kFormCapped = 1, kFormCompact = 2;
+
+template <bool kSmemArena, bool kSmemTable, bool kPersistent, int kLean = 0, int kForm = kFormAny>
 __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ? 512 : 1024),
-                                  kLean == 2 ? 12 : kLean ? 8 : 1) qtb_network_kernel(
+                                  kLean == 2 ? 12 : kLean ? 8 : kForm == kFormAny ? 1 : 2) qtb_network_kernel(
     const Job* __restrict__ jobs, const RunArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
@@ -889,7 +898,7 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
         // a network with element records needs no blob (shared table and
         // arena only); otherwise blob_capacity 0: the launch reads plan
         // blobs from global memory
-        const bool records = kSmemArena && kSmemTable && a.recs != nullptr && net.rec_words != 0;
+        const bool records = kForm == kFormCompact || (kSmemArena && kSmemTable && a.recs != nullptr && net.rec_words != 0);
         const bool staged = !records && a.blob_capacity != 0;
         if (net.arena_elems > a.arena_capacity || (staged && net.blob_bytes > a.blob_capacity)) {
             if (threadIdx.x == 0)
@@ -914,7 +923,7 @@ __global__ void __launch_bounds__(kLean == 2 ? 96 : kLean ? 128 : (kPersistent ?
             staged ? blob : reinterpret_cast<const unsigned char*>(a.blobs + net.blob_off16);
         float2 term;
         if (!records) term = contract_network<kSmemTable>(net, nblob, table, arena);
-        else if (net.rec_format == kRecCompact)
+        else if (kForm == kFormCompact || net.rec_format == kRecCompact)
             term = contract_records_compact(net, a.recs + net.rec_off, stable, arena, s_head, start);
         else term = contract_records(net, a.recs + net.rec_off, stable, arena, s_head, start);
         if (threadIdx.x == 0) {
@@ -1931,6 +1940,8 @@ struct LaunchClass {
     int lean;               // persistent, registers capped: 1 = 128 threads (8 CTAs per SM), 2 = 96 (12)
     bool warp;              // persistent, every warp takes networks (qtb_warp_network_kernel)
     bool records;           // networks with element records contract from them
+    bool compact;           // every network contracts from compact element records
+    int form;               // kForm* of a persistent launch (persistent_grid)
     int grid;               // CTAs (= n_jobs unless persistent)
     uint32_t capacity;      // arena elements per CTA
     uint32_t blob_capacity; // plan-blob bytes per CTA
@@ -2062,6 +2073,19 @@ static void launch_one(const LaunchClass& lc, const Job* jobs, const RunArgs& a,
         qtb_warp_network_kernel<kT><<<lc.grid, lc.threads, lc.smem_bytes, st>>>(jobs, a);
         return;
     }
+    if constexpr (kA && kT) {
+        if (lc.compact && lc.lean == 2) {
+            qtb_network_kernel<true, true, true, 2, kFormCompact>
+                <<<lc.grid, kLean12Threads, lc.smem_bytes, st>>>(jobs, a);
+            return;
+        }
+        if (lc.form != kFormAny && lc.persistent && !lc.lean) {
+            const auto kernel = lc.form == kFormCompact ? qtb_network_kernel<true, true, true, 0, kFormCompact>
+                                                        : qtb_network_kernel<true, true, true, 0, kFormCapped>;
+            kernel<<<lc.grid, lc.threads, lc.smem_bytes, st>>>(jobs, a);
+            return;
+        }
+    }
     if constexpr (kA) {
         if (lc.lean == 2) {
             qtb_network_kernel<true, kT, true, 2><<<lc.grid, kLean12Threads, lc.smem_bytes, st>>>(jobs, a);
@@ -2089,9 +2113,9 @@ static void launch_class(const LaunchClass& lc, bool smem_table, const Job* jobs
     }
 }
 
-template <bool kA, bool kT, bool kP, int kL = 0>
+template <bool kA, bool kT, bool kP, int kL = 0, int kF = kFormAny>
 static cudaError_t allow_smem() {
-    return cudaFuncSetAttribute(qtb_network_kernel<kA, kT, kP, kL>,
+    return cudaFuncSetAttribute(qtb_network_kernel<kA, kT, kP, kL, kF>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
 }
 
@@ -2108,6 +2132,9 @@ static int allow_all_smem() {
     QTB_CUDA((allow_smem<true, false, true, 1>()));
     QTB_CUDA((allow_smem<true, true, true, 2>()));
     QTB_CUDA((allow_smem<true, false, true, 2>()));
+    QTB_CUDA((allow_smem<true, true, true, 0, kFormCapped>()));
+    QTB_CUDA((allow_smem<true, true, true, 0, kFormCompact>()));
+    QTB_CUDA((allow_smem<true, true, true, 2, kFormCompact>()));
     QTB_CUDA(cudaFuncSetAttribute(qtb_warp_network_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kSmemLimitBytes));
     QTB_CUDA(cudaFuncSetAttribute(qtb_warp_network_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2116,8 +2143,17 @@ static int allow_all_smem() {
     return QTB_OK;
 }
 
-// Resident CTAs of a persistent launch class on the whole GPU.
-static int persistent_grid(const LaunchClass& lc, bool smem_table, int* grid) {
+// Resident CTAs of a persistent launch class on the whole GPU, and the form of
+// its kernel: the one of at most 64 registers where that holds more CTAs and
+// every CTA of kFormAny would take two networks or more.  Whole calls, kFormAny
+// against it, compact records: N=1000 p=3 (another graph than below) at 128
+// threads 53.2 / 46.9 us, N=700 p=2 at 256 46 / 35; all formats: N=1000 p=3 at
+// 256 74.2 / 56.3 and at 512 115 / 81, N=700 p=3 at 256 59 / 48, N=250 p=3 at
+// 512 50.4 / 43.7, N=200 48.5 / 46.6.  Below the line: N=150 at 512 (225
+// networks, 148 CTAs) 44.4 / 46.1, N=100 45.3 / 47.0; and where shared memory
+// holds as few, N=1000 at 128, 52.5 / 54.8.  Autotuned calls over 50 graphs of
+// 1 to 3 layers, geometric mean: 40.7 us with kFormAny alone, 40.3 with all.
+static int persistent_grid(LaunchClass& lc, bool smem_table, int* grid) {
     int per_sm = 0, sms = 0, dev = 0;
     QTB_CUDA(cudaGetDevice(&dev));
     QTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2133,7 +2169,10 @@ static int persistent_grid(const LaunchClass& lc, bool smem_table, int* grid) {
         *grid = std::max(1, std::min((lc.n_jobs + warps - 1) / warps, std::max(1, per_sm) * sms));
         return QTB_OK;
     } else if (lc.lean == 2) {
-        if (smem_table)
+        if (lc.compact)
+            QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &per_sm, qtb_network_kernel<true, true, true, 2, kFormCompact>, kLean12Threads, lc.smem_bytes));
+        else if (smem_table)
             QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &per_sm, qtb_network_kernel<true, true, true, 2>, kLean12Threads, lc.smem_bytes));
         else
@@ -2147,12 +2186,23 @@ static int persistent_grid(const LaunchClass& lc, bool smem_table, int* grid) {
             QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &per_sm, qtb_network_kernel<true, false, true, 1>, kLeanThreads, lc.smem_bytes));
     } else if (lc.smem) {
-        if (smem_table)
+        if (smem_table) {
+            int dense = 0;
             QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &per_sm, qtb_network_kernel<true, true, true>, lc.threads, lc.smem_bytes));
-        else
+            QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &dense, lc.compact ? qtb_network_kernel<true, true, true, 0, kFormCompact>
+                                   : qtb_network_kernel<true, true, true, 0, kFormCapped>,
+                lc.threads, lc.smem_bytes));
+            lc.form = kFormAny;
+            if (dense > per_sm && lc.n_jobs >= 2 * per_sm * sms) {
+                lc.form = lc.compact ? kFormCompact : kFormCapped;
+                per_sm = dense;
+            }
+        } else {
             QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &per_sm, qtb_network_kernel<true, false, true>, lc.threads, lc.smem_bytes));
+        }
     } else {
         per_sm = 1;
     }
@@ -2645,6 +2695,7 @@ static int build_run(qtb_plan* plan, int32_t first, int32_t count, float2* terms
         lc.smem = smem;
         lc.persistent = persistent;
         lc.records = smem && with_recs && recs;
+        lc.compact = lc.records;
         lc.job_offset = jobs.size();
         lc.n_jobs = (int)m.size();
         lc.grid = lc.n_jobs;
@@ -2653,11 +2704,13 @@ static int build_run(qtb_plan* plan, int32_t first, int32_t count, float2* terms
             cap = std::max(cap, plan->druns[i].arena_elems);
             blob = std::max(blob, staged_blob(plan->druns[i], lc.records));
             maxe = std::max(maxe, plan->druns[i].max_elems);
+            lc.compact = lc.compact && plan->druns[i].rec_words != 0 && plan->druns[i].rec_format == kRecCompact;
             Job j{};
             j.net = plan->druns[i];
             j.term = terms + (i - first);
             jobs.push_back(j);
         }
+        lc.form = kFormAny;
         lc.capacity = (cap + 3u) & ~3u;
         // a global-arena class whose largest blob does not fit shared memory
         // reads every member's blob from global memory (capacity 0)
