@@ -98,7 +98,8 @@ int qtb_bucket_c64(const qtb_bucket_desc* desc, const void* const* inputs,
  * cores in FP32.  scratch (qtb_contract_sum_scratch_bytes for the same
  * shape and mode) holds the split operands; its first 4 bytes are a status
  * word, 0 after a good run, 2 when a staging copy or the MMAs did not
- * complete within the kernel's bounded wait.                              */
+ * complete within the kernel's bounded wait (the outputs of the tiles
+ * concerned are then not written).                                        */
 int qtb_contract_outer_c64(const void* a, const void* b, void* c, int64_t n, int64_t m, int64_t k,
                            void* stream);
 int qtb_contract_sum_scratch_bytes(int64_t K, int64_t F, int64_t M, int64_t N, int32_t mode, size_t* bytes);

@@ -53,7 +53,7 @@ namespace qtb {
 // (1.8 TB/s of 6.5 for the outer product, 1.2 TB/s for K = 2).  Rows in a
 // block share the load of their b, and with kPairs (N even, 16-byte aligned
 // pointers) two columns load and store 16 bytes.  256 x 256 x 256 outer
-// product: 73.7 -> 23.6 us; K = 2, F = 64, M = N = 512: 116 -> 24.9 us (134 MB
+// product: 73.6 -> 23.3 us; K = 2, F = 64, M = N = 512: 116 -> 26.7 us (134 MB
 // written; a memset of it takes 20.6 us).
 // I: 32-bit indices, or 64-bit where a dimension needs them.
 template <typename I>
@@ -95,11 +95,16 @@ constexpr int kFlatThreads = 256;
 constexpr int kFlatBlocksPerSm = 4;   // all resident at 64 registers (48 spill: K = 2 41 us; 74 and 8 per SM: 42)
 constexpr int kFlatRows = 4;
 // Outputs from here on are stored evict-first, when pairs of columns are (8-byte
-// stores were not measured and stay plain).  Plain against evict-first, and
-// each with a reduction of the output behind it: K = 2 into 128 MiB 33.1
-// against 24.9 us and 67.9 / 68.1, the outer product 24.8 against 23.7 and
-// 60.0 / 59.8; at 104 MiB 26.8 against 21.0 and 54.6 / 55.2; at 64 MiB, where
-// a reader finds the output in L2, 18.9 against 14.6 but 33.1 / 39.2.
+// stores were not measured and stay plain).  What is gained is write-back that
+// no longer waits for lines in L2 to be evicted: a call alone, or followed by
+// work on other data, is faster, a reader of the output right behind it finds
+// as little in L2 either way.  Plain against evict-first, and each with a
+// reduction of the output behind it: K = 2 into 128 MiB 33.1 against 24.9 us
+// and 67.9 / 68.1, the outer product 24.8 against 23.7 and 60.0 / 59.8; around
+// the line K = 2 takes 26.2 and 27.3 us (100.8 and 103.8 MiB, plain), 22.2
+// and 23.2 (104.8 and 111.8, evict-first), with the reduction 53.9, 55.2, 55.5
+// and 59.8.  At 64 MiB, where a reader finds the output in L2, 18.9 against
+// 14.6 but 33.1 / 39.2.
 constexpr uint64_t kFlatStreamBytes = 104ull << 20;
 static bool flat_stream(uint64_t outputs) { return outputs * sizeof(float2) >= kFlatStreamBytes; }
 
@@ -445,7 +450,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 // cycles per 8 k, read 72 KB of operands and see 40 KB written: 875 cycles at
 // 128 bytes each (measured about 1100).  128 x 64 tiles with B stored as both
 // [Br | Bi] and [-Bi | Br] also pulled 32 KB per 384 cycles through L2.
-// K=1024, F=2, M=N=1024: 165 -> 106 us; K=500, F=3, M=333, N=190: 71 -> 23 us
+// K=1024, F=2, M=N=1024: 165 -> 112 us per call; K=500, F=3, M=333, N=190: 71 -> 23 us
 // (4 CTAs per tile in place of 27 serial ones).  Measured and not kept: B as
 // [Br | Bi] with the negative products through the descriptor's negate-A bit
 // (32 KB per tile but N = 128 MMAs, 128 operand bytes per cycle: 116 us).

@@ -2833,11 +2833,12 @@ static int build_run(qtb_plan* plan, int32_t first, int32_t count, float2* terms
             rc->wclasses.push_back(lc);
         }
     }
-    // networks too large for shared memory run as whole-GPU waves (K4);
+    // networks too large for shared memory run in waves (K4);
     // QTB_CLUSTER_MAX_ELEMS=<elements> in the environment runs those whose
     // arena is at most that as one thread-block cluster each (K5) instead.
-    // Waves are the default: on N=256 p=4 and Erdos-Renyi N=400 p=3 they
-    // took 0.71 and 2.06 ms, clusters of 2-16 CTAs 0.74-1.30 and 3.4-9.8 ms.
+    // Waves are the default: on N=256 p=4 and Erdos-Renyi N=400 p=3 (not the
+    // graphs at qtb_wide_kernel) they take 0.31 and 0.74 ms, clusters of 8 and
+    // 16 CTAs 0.78 and 1.31 ms, 2.62 and 2.39 ms.
     std::vector<int32_t> wave_nets, cl_nets;
     uint64_t cl_max = 0;
     if (const char* env = std::getenv("QTB_CLUSTER_MAX_ELEMS")) cl_max = std::strtoull(env, nullptr, 10);

@@ -94,8 +94,9 @@ class CompiledGraph:
                       self.terms, self.energy, self.scratch, stream.cuda_stream)
 
     def launch_plain(self, params_dev=None, stream=None):
-        """The plain path, asynchronously: one bucket-kernel launch per bucket
-        (the drop-in backend's process_bucket), networks in sequence,
+        """The plain path, asynchronously: one launch of the simple bucket
+        kernel per bucket, whatever its size (it shares no code with the wide
+        waves, which are compared with it), networks in sequence,
         intermediates in global memory; results in ``self.terms`` and
         ``self.energy`` as with ``launch``."""
         stream = torch.cuda.current_stream(self.device) if stream is None else stream

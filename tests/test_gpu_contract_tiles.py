@@ -1,6 +1,7 @@
-"""Edges of the tensor-core contract-sum's tiles: one and two column tiles of
-either width, rows past the last tile, K split over 1 to 8 CTAs with uneven
-parts, odd N (8-byte stores) and a C that is only 8-byte aligned.  The bar is
+"""Edges of the tensor-core contract-sum's 128 x 64 tiles (the wider ones are in
+test_gpu_contract_wide_tiles.py): one and more column tiles, rows past the
+last tile, K split over 1 to 8 CTAs with even and uneven parts, odd N (8-byte
+stores) and a C that is only 8-byte aligned.  The bar is
 the repository's for this path: 1e-5 of the largest output magnitude."""
 import numpy as np
 import pytest
@@ -16,7 +17,7 @@ TOL = 1e-5
 @pytest.mark.parametrize('K,F,M,N', [
     (32, 1, 1, 1), (33, 1, 128, 64), (64, 1, 129, 65), (160, 2, 127, 128), (257, 1, 64, 129),
     (300, 40, 130, 130),        # more tiles than SMs
-    (1000, 1, 100, 96),         # one tile, K in eight uneven parts
+    (1000, 1, 100, 96),         # two tiles, K in eight parts
     (544, 2, 300, 250),
 ])
 @pytest.mark.parametrize('shift', [0, 1])
